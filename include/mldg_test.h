@@ -41,7 +41,19 @@ int mldg_rep_plan_check(const mldg_csr *L, const mldg_csr *U, const double *d, c
 int mldg_blk_plan_check(const mldg_csr *T, int upper, const double *scale, const double *rhs, double *t,
                         int nblocks, int fp32, long long *stats);
 
-/* Polls a sentinel wait of the sync-free and ELL triangular solves makes
+/* Builds the grouped plan (k_trsv_grp) of the strictly triangular factor T
+ * (0-based CSR, n x n; upper != 0: an upper factor) for ncols columns (a power
+ * of two up to 32), exactly as mldg_finalize would, and replays its warp tasks
+ * in ticket order on one right-hand side: every position written once, every
+ * index in range, every dependency written by an earlier group.
+ * t = (I + T)^{-1} (scale o rhs) (scale may be NULL).  budget, row, growth:
+ * entries per group, entries per row and bound on a row of the inverted
+ * blocks, 0 for the defaults.  stats[4]: violations, dependency levels,
+ * groups, entries.  Returns MLDG_SUCCESS or an error code. */
+int mldg_grp_plan_check(const mldg_csr *T, int upper, const double *scale, const double *rhs, double *t,
+                        int ncols, long long budget, int row, double growth, int fp32, long long *stats);
+
+/* Polls a sentinel wait of the sync-free, ELL and grouped triangular solves makes
  * before it gives up with MLDG_ERR_TIMEOUT, on `device`; polls < 0 restores
  * the default (2^22).  A test lowers it (0: give up at the first poll that
  * finds a dependency not yet written) to make a solve's waits run out on

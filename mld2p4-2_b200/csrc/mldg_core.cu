@@ -33,9 +33,11 @@
 #include "mldg_kernels.cuh"
 #include "mldg_multi.cuh"
 #include "mldg_tri.h"
+#include "mldg_trigrp.h"
 #include "mldg_trsv_win.cuh"
 #include "mldg_trsv_rep.cuh"
 #include "mldg_trsv_blk.cuh"
+#include "mldg_trsv_grp.cuh"
 #include "mldg_ilu0.cuh"
 #include "mldg_spgemm.cuh"
 #include "mldg_spmv_stg.cuh"
@@ -165,10 +167,14 @@ struct Arena {
     return (T *)p;
   }
   template <typename T>
-  T *upload(const std::vector<T> &v) {
-    T *p = alloc<T>(v.size());
-    if (!v.empty()) MLDG_CUDA(cudaMemcpy(p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));
+  T *upload(const T *v, size_t n) {
+    T *p = alloc<T>(n);
+    if (n) MLDG_CUDA(cudaMemcpy(p, v, n * sizeof(T), cudaMemcpyHostToDevice));
     return p;
+  }
+  template <typename T>
+  T *upload(const std::vector<T> &v) {
+    return upload(v.data(), v.size());
   }
   void release() {
     for (void *p : ptrs) cudaFree(p);
@@ -447,6 +453,167 @@ struct DBlk {
   int2 *sdesc = nullptr;
   uint4 *plan = nullptr;
   int *ticket = nullptr;
+};
+
+// Grouped solve: entries of V and W per group, entries of a row, the bound on a
+// row of W, and the widest block of columns.  A group's entries should stream
+// in about the time of its hand-off, which takes longer the more warps take
+// part: n/5 entries between these limits (solve pair at idim=40, 64,000 rows:
+// 86 us with 50,000 and 100,000, 98 us with 200,000; idim=101, 1,030,301 rows:
+// 333 us with 200,000, 408 us with 100,000).  Blocks above eight columns keep
+// the ELL solve: their gathers move 32 values an entry, so the fill costs more
+// than the hand-offs it saves (32 columns at idim=64: 250 us a solve against 178).
+constexpr int64_t kGrpBudgetMin = 50000, kGrpBudgetMax = 200000;
+constexpr int kGrpRow = 512;
+constexpr double kGrpGrowth = 64.0;
+constexpr int kGrpCols = 8;
+static int64_t grp_budget(int n, int K) {
+  return K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
+}
+// columns of one task: a 32-byte sector of a row's K values
+template <typename T>
+constexpr int grp_cols(int K) {
+  return K < (int)(32 / sizeof(T)) ? K : (int)(32 / sizeof(T));
+}
+
+// original row of every position, and the dependencies as positions
+static void grp_positions(int n, bool rev, const std::vector<int> &prow, const std::vector<int> &pja,
+                          std::vector<int> &orig, std::vector<int> &dep) {
+  std::vector<int> pos((size_t)n);
+  orig.resize((size_t)n);
+  dep.resize(pja.size());
+  for (int p = 0; p < n; ++p) {
+    pos[prow[p]] = p;
+    orig[p] = rev ? n - 1 - prow[p] : prow[p];
+  }
+#pragma omp parallel for schedule(static, 4096)
+  for (int64_t k = 0; k < (int64_t)dep.size(); ++k) dep[k] = pos[pja[k]];
+}
+
+// Warp tasks of a grouped plan (layout: mldg_trsv_grp.cuh).
+template <typename T>
+struct GrpTasks {
+  std::vector<int4> desc;
+  std::unique_ptr<int4[]> idx;  // left uninitialised until the threads that fill it touch it
+  std::unique_ptr<T[]> val;
+  int64_t slots = 0;  // entries stored, padding included
+};
+// wcol(c), wscale(c): index in b and factor of W's column position c; false
+// when the slots outgrow the descriptors
+template <typename T, typename FC, typename FS>
+static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, GrpTasks<T> &out) {
+  const int R = 32 / KC, ng = (int)g.gptr.size() - 1;
+  auto len = [&](int p) { return (int64_t)std::max(g.row[p].nv, g.row[p].nw); };
+  int64_t at = 0;  // slot groups (one int4 of indices each)
+  for (int b = 0; b < ng; ++b)
+    for (int p = g.gptr[b]; p < g.gptr[b + 1];) {
+      // lanes per (row, column) so that every row of the task is one pass of
+      // eight entries a lane; rows lengthen along a group, so a longer row
+      // ahead widens the task's lanes and narrows the task
+      int lt = 0, rows = 1;
+      auto fits = [&](int64_t l) { return l <= (8 << lt) || (2 << lt) > R; };
+      while (!fits(len(p))) ++lt;
+      while (rows < (R >> lt) && p + rows < g.gptr[b + 1]) {
+        const int keep = lt;
+        while (!fits(len(p + rows))) ++lt;
+        if (rows + 1 > (R >> lt)) {
+          lt = keep;
+          break;
+        }
+        ++rows;
+      }
+      int64_t nw = 0, nv = 0;
+      for (int r = p; r < p + rows; ++r) {
+        nw = std::max<int64_t>(nw, g.row[r].nw);
+        nv = std::max<int64_t>(nv, g.row[r].nv);
+      }
+      nw = (nw + (4 << lt) - 1) / (4 << lt);
+      nv = (nv + (4 << lt) - 1) / (4 << lt);
+      if (nw > 0x7fff || nv > 0x7fff || at + (nw + nv) * R >= INT32_MAX) return false;
+      out.desc.push_back(make_int4((int)at, (int)(nw | nv << 16), p, rows << 8 | lt));
+      at += (nw + nv) * R;
+      p += rows;
+    }
+  out.idx.reset(new int4[(size_t)std::max<int64_t>(at, 1)]);
+  out.val.reset(new T[(size_t)std::max<int64_t>(4 * at, 1)]);
+#pragma omp parallel for schedule(static, 64)
+  for (int64_t k = 0; k < (int64_t)out.desc.size(); ++k) {
+    const int4 d = out.desc[k];
+    const int lt = d.w & 255, rows = d.w >> 8, tpr = 1 << lt;
+    const int64_t end = d.x + (int64_t)((d.y & 0xffff) + (d.y >> 16)) * R;
+    std::fill(out.idx.get() + d.x, out.idx.get() + end, make_int4(-1, -1, -1, -1));
+    std::fill(out.val.get() + 4 * (int64_t)d.x, out.val.get() + 4 * end, T(0));
+    for (int r = 0; r < rows; ++r) {
+      // entry e of the row: slot e / tpr of lane e % tpr
+      auto put = [&](int64_t base, int64_t e, int c, double v) {
+        const int64_t slot = e >> lt, q = base + (slot >> 2) * R + r * tpr + (e & (tpr - 1));
+        (&out.idx[(size_t)q].x)[slot & 3] = c;
+        out.val[(size_t)(4 * q + (slot & 3))] = (T)v;
+      };
+      const GroupRow &gr = g.row[d.z + r];
+      for (int e = 0; e < gr.nw; ++e) put(d.x, e, wcol(gr.w[e].col), gr.w[e].val * wscale(gr.w[e].col));
+      for (int e = 0; e < gr.nv; ++e) put(d.x + (int64_t)(d.y & 0xffff) * R, e, gr.v[e].col, gr.v[e].val);
+    }
+  }
+  out.slots = 4 * at;
+  return true;
+}
+
+// Replays a grouped plan's tasks in ticket order: every position written
+// once, every index in range, every dependency written by an earlier group.
+// Returns the number of violations; x solves the factor for rhs.
+template <typename T>
+static int64_t grp_emulate(const TriGroups &g, const GrpTasks<T> &m, int KC, const std::vector<double> &rhs,
+                           std::vector<double> &x) {
+  const int n = g.gptr.back(), R = 32 / KC;
+  int64_t bad = 0;
+  x.assign((size_t)n, 0.0);
+  std::vector<char> done((size_t)n, 0);
+  size_t grp = 0;
+  for (const int4 &d : m.desc) {
+    const int lt = d.w & 255, rows = d.w >> 8, tpr = 1 << lt, nw = d.y & 0xffff, nv = d.y >> 16;
+    while (grp + 1 < g.gptr.size() && d.z >= g.gptr[grp + 1]) ++grp;
+    if (rows < 1 || rows * tpr > R || d.z < 0 || d.z + rows > g.gptr[grp + 1] || d.x < 0 || nv < 0 ||
+        4 * (d.x + (int64_t)(nw + nv) * R) > m.slots) {
+      ++bad;
+      continue;
+    }
+    for (int r = 0; r < rows; ++r) {
+      T acc = T(0);
+      for (int sub = 0; sub < tpr; ++sub)
+        for (int s = 0; s < nw + nv; ++s) {
+          const size_t q = (size_t)d.x + (size_t)s * R + r * tpr + sub;
+          for (int e = 0; e < 4; ++e) {
+            const int j = (&m.idx[q].x)[e];
+            if (j < 0) continue;
+            if (j >= n || (s >= nw && (j >= g.gptr[grp] || !done[j]))) {
+              ++bad;
+              continue;
+            }
+            if (s < nw)
+              acc += m.val[4 * q + e] * (T)rhs[j];
+            else
+              acc -= m.val[4 * q + e] * (T)x[j];
+          }
+        }
+      const int p = d.z + r;
+      bad += done[p];
+      done[p] = 1;
+      x[p] = (double)acc;
+    }
+  }
+  for (int p = 0; p < n; ++p) bad += !done[p];
+  return bad;
+}
+
+// Plan of the grouped solve (k_trsv_grp) for one triangular factor and one
+// column width.
+template <typename T>
+struct DGrp {
+  int n = 0, grid = 0;
+  GrpMat<T> m{};
+  int64_t slots = 0;  // stored entries, padding included
+  int *orig = nullptr;
 };
 
 static int pick_tpr(int64_t nnz, int nr) {
@@ -758,6 +925,14 @@ static void kdispatch(int K, F &&f) {
   }
 }
 // the ELL triangular solve also serves the single-vector V-cycle (K = 1)
+// the same with one column (K = 1) too
+template <typename F>
+static void kdispatch1(int K, F &&f) {
+  if (K == 1)
+    f(std::integral_constant<int, 1>());
+  else
+    kdispatch(K, f);
+}
 template <typename F>
 static void kdispatch_ell(int K, F &&f) {
   if (K == 1)
@@ -1007,6 +1182,19 @@ struct EngineT : Engine {
     // (blk) when the autotuner finds them fastest
     bool blk = false, blk_ok = false;
     DBlk<T> kL, kU, kUt, kLt;
+    // grouped solves (k_trsv_grp) of every factor, per log2 of the column
+    // width.  A recorded cycle's s-th solve on the level writes x[s % ring] and
+    // resets x[(s + ring / 2) % ring]: by then the solve that read it is over
+    // (ring 4 for ILU(0) pairs, whose second solve reads the first's; 2 for the
+    // single Gauss-Seidel solves).  seq counts the cycle's solves.
+    bool grp = false;
+    std::vector<double> h_d;  // d on the host: folded into W of the scaled solves
+    struct Grp {
+      DGrp<T> L, U, Ut, Lt;
+      T *x[4] = {};
+      int *ctr = nullptr;  // one ticket counter per buffer
+      int ring = 4, seq = 0;
+    } g[6];
     // coarsest level: explicit inverse of its ILU(0) factorisation (and its transpose)
     T *minv = nullptr, *minvT = nullptr;
     T *rp0 = nullptr, *rp1 = nullptr;  // right-hand sides in position order
@@ -1300,7 +1488,7 @@ struct EngineT : Engine {
     MLDG_CUDA(cudaEventCreate(&e1));
     for (auto &L : lv) {
       const bool gs = L.kind == MLDG_SMOOTHER_FBGS;
-      if ((L.kind != MLDG_SMOOTHER_BJAC && !gs) || L.minv || !L.L.ell[0].ok || !L.U.ell[0].ok ||
+      if ((L.kind != MLDG_SMOOTHER_BJAC && !gs) || L.minv || L.grp || !L.L.ell[0].ok || !L.U.ell[0].ok ||
           (!gs && (!L.Ut.ell[0].ok || !L.Lt.ell[0].ok)))
         continue;
       // the timed operation: the ILU solve pair, or a forward + backward GS solve
@@ -1452,6 +1640,74 @@ struct EngineT : Engine {
         w.nnz * (int64_t)(sizeof(T) + 4) + 4 * ((int64_t)w.n + 1) + vec);
   }
 
+  // One grouped solve x = (factor)^{-1} (scale o rhs) in position order, the
+  // scaling and rhs's order folded into W's columns; out (original order)
+  // = x + beta*out when given.  Returns x.
+  const T *gsolve(typename Lev::Grp &G, const DGrp<T> &g, int Kw, int64_t nnz, const T *rhs, T *out, T beta) {
+    const int s = G.seq % G.ring, r = (G.seq + G.ring / 2) % G.ring;
+    ++G.seq;
+    GrpArgs<T> a;
+    a.m = g.m;
+    a.K = Kw;
+    a.ncb = Kw / grp_cols<T>(Kw);
+    a.rhs = rhs;
+    a.x = G.x[s];
+    a.reset = G.x[r];
+    a.orig = g.orig;
+    a.out = out;
+    a.alpha = T(1);
+    a.beta = beta;
+    a.ctr = G.ctr + 32 * s;
+    a.ctr_reset = G.ctr + 32 * r;
+    a.err = err;
+    begin(MLDG_KERNEL_TRSV);
+    grp_dispatch(Kw, [&](auto kc) { kl(k_trsv_grp<T, decltype(kc)::value>, g.grid, 256, a); });
+    const int64_t vec = (int64_t)g.n * Kw * (int64_t)sizeof(T) * (3 + (out ? 1 + (beta != T(0)) : 0));
+    end(g.slots * (int64_t)(sizeof(T) + 4) + 16 * (int64_t)g.m.ntask + vec,
+        nnz * (int64_t)(sizeof(T) + 4) + 4 * (2 * (int64_t)g.n + 1) + vec);
+    return G.x[s];
+  }
+  // K dispatched by the columns of a task
+  template <typename F>
+  static void grp_dispatch(int Kw, F &&f) {
+    switch (grp_cols<T>(Kw)) {
+      case 1: f(std::integral_constant<int, 1>()); break;
+      case 2: f(std::integral_constant<int, 2>()); break;
+      case 4: f(std::integral_constant<int, 4>()); break;
+      default: f(std::integral_constant<int, (int)(32 / sizeof(T))>());
+    }
+  }
+  void gpair(Lev &L, int Kw, char trans, const T *x, T beta, T *y) {
+    auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
+    if (trans == 'N') {
+      const T *z = gsolve(G, G.L, Kw, L.nnz_l, x, nullptr, T(0));
+      gsolve(G, G.U, Kw, L.nnz_u, z, y, beta);
+    } else {
+      const T *z = gsolve(G, G.Ut, Kw, L.nnz_u, x, nullptr, T(0));
+      gsolve(G, G.Lt, Kw, L.nnz_l, z, y, beta);
+    }
+  }
+  // End of a recorded cycle: the next one starts with x[0] (and x[1] for
+  // pairs) at the sentinel and the counters at zero; put back those that the
+  // last solves left used (none when a level makes a multiple of ring solves).
+  void end_grp(int Kw) {
+    const int ki = Kw == 1 ? 0 : ilog2(Kw);
+    for (auto &L : lv) {
+      auto &G = L.g[ki];
+      if (!L.grp || !G.seq) continue;
+      for (int b = 0; b < G.ring / 2; ++b)
+        for (int s = std::max(0, G.seq - G.ring / 2); s < G.seq; ++s)
+          if (s % G.ring == b) {
+            begin(MLDG_KERNEL_VEC);
+            const int64_t nn = (int64_t)L.n * Kw;
+            kl(k_fill<T>, blocks_for(nn), 256, (int)nn, Sentinel<T>::value(), G.x[b]);
+            end(nn * (int64_t)sizeof(T));
+            kl(k_fill<int>, 1, 32, 1, 0, G.ctr + 32 * b);
+          }
+      G.seq = 0;
+    }
+  }
+
   // ILU solver apply: y = alpha*U^{-1}(d o L^{-1} x) + beta*y, or the 'T' form
   void ilu_apply(Lev &L, char trans, const T *x, T beta, T *y) {
     if (L.minv) {
@@ -1462,6 +1718,10 @@ struct EngineT : Engine {
       end((int64_t)L.n * L.n * sizeof(T) + (int64_t)L.n * sizeof(T) * (2 + (beta != T(0))),
           (L.nnz_l + L.nnz_u) * (int64_t)(sizeof(T) + 4) + 8 * ((int64_t)L.n + 1) +
               (int64_t)L.n * sizeof(T) * (3 + (beta != T(0))));
+      return;
+    }
+    if (L.grp) {
+      gpair(L, 1, trans, x, beta, y);
       return;
     }
     if (L.blk) {
@@ -1525,6 +1785,11 @@ struct EngineT : Engine {
               (int64_t)L.n * sizeof(T) * (3 + (beta != T(0))));
       return;
     }
+    if (L.grp) {
+      auto &G = L.g[0];
+      gsolve(G, backward ? G.U : G.L, 1, backward ? L.nnz_u : L.nnz_l, rhs, out, beta);
+      return;
+    }
     const DTri<T> &t = backward ? L.U : L.L;
     T *cur = L.gflip ? L.bufB : L.bufA, *other = L.gflip ? L.bufA : L.bufB;
     L.gflip ^= 1;
@@ -1552,6 +1817,7 @@ struct EngineT : Engine {
       for (DRep<T> *r : {&L.rL, &L.rU, &L.rUt, &L.rLt}) refill(r->xp, (int64_t)r->n + 8);
       for (DBlk<T> *k : {&L.kL, &L.kU, &L.kUt, &L.kLt})
         if (k->ticket) MLDG_CUDA(cudaMemsetAsync(k->ticket, 0, 2 * sizeof(int), st));
+      for (int Kw = 1; Kw <= 32; Kw *= 2) reset_grp(L, Kw);
       L.gflip = 0;
       L.gflip_m = 0;
     }
@@ -1910,6 +2176,81 @@ struct EngineT : Engine {
   }
   int64_t nk(int n) const { return (int64_t)n * K; }
 
+  // Grouped plan of factor t for Kw columns: rhs_pos (original row -> index of
+  // the right-hand side; null: original order), scale (by original row, or
+  // null); pos_out: original row -> position.
+  bool build_grp_factor(Arena &ar, const DTri<T> &t, int Kw, const std::vector<int> *rhs_pos,
+                        const std::vector<double> *scale, DGrp<T> &g, std::vector<int> *pos_out) {
+    const int n = t.n, KC = grp_cols<T>(Kw);
+    std::vector<int> orig, dep;
+    grp_positions(n, t.rev != 0, t.h_prow, t.h_pja, orig, dep);
+    int64_t budget = grp_budget(n, Kw);
+    if (const char *e = std::getenv("MLDG_GRP_B")) budget = std::max(1, std::atoi(e));
+    TriGroups pl;
+    build_tri_groups(t.h_lvl, t.h_pirp, dep, t.h_pval, budget, kGrpRow, kGrpGrowth, &pl);
+    GrpTasks<T> tk;
+    if (!grp_tasks<T>(
+            pl, KC, [&](int c) { return rhs_pos ? (*rhs_pos)[orig[c]] : orig[c]; },
+            [&](int c) { return scale ? (*scale)[orig[c]] : 1.0; }, tk))
+      return false;
+    g.n = n;
+    g.slots = tk.slots;
+    g.m.ntask = (int)tk.desc.size();
+    g.m.desc = ar.upload(tk.desc);
+    g.m.idx = ar.upload(tk.idx.get(), (size_t)tk.slots / 4);
+    g.m.val = ar.upload(tk.val.get(), (size_t)tk.slots);
+    g.orig = ar.upload(orig);
+    // warps in flight: eight groups' tasks, so that a group's tasks have their
+    // entries and older values loaded when the group before it is finished
+    // (idim=101 level 0: 822 us for four solves with four groups, 680 with eight)
+    int nb = 0;
+    grp_dispatch(Kw, [&](auto kc) {
+      MLDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trsv_grp<T, decltype(kc)::value>, 256, 0));
+    });
+    const int ng = (int)pl.gptr.size() - 1;
+    const int64_t ntask = (int64_t)g.m.ntask * (Kw / KC), per = (ntask + ng - 1) / ng;
+    const int64_t warps = std::max<int64_t>(32, std::min<int64_t>(8 * per, ntask));
+    g.grid = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, (int64_t)std::max(nb, 1) * nsm));
+    if (std::getenv("MLDG_VERBOSE"))
+      std::fprintf(stderr, "mldg: grp K=%d n=%d levels=%d groups=%d entries %lld slots %lld tasks %d grid %d occ %d\n", Kw, n,
+                   t.nlevels, ng, (long long)pl.entries, (long long)g.slots, g.m.ntask, g.grid, nb);
+    if (pos_out) {
+      pos_out->resize((size_t)n);
+      for (int p = 0; p < n; ++p) (*pos_out)[orig[p]] = p;
+    }
+    return true;
+  }
+  // the grouped plans and work vectors of a level for Kw columns
+  bool build_grp(Lev &L, int Kw, Arena &ar) {
+    auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
+    bool ok;
+    if (L.kind == MLDG_SMOOTHER_FBGS) {
+      G.ring = 2;
+      ok = build_grp_factor(ar, L.L, Kw, nullptr, &L.h_d, G.L, nullptr) &&
+           build_grp_factor(ar, L.U, Kw, nullptr, &L.h_d, G.U, nullptr);
+    } else {
+      std::vector<int> pos;
+      ok = build_grp_factor(ar, L.L, Kw, nullptr, nullptr, G.L, &pos) &&
+           build_grp_factor(ar, L.U, Kw, &pos, &L.h_d, G.U, nullptr) &&
+           build_grp_factor(ar, L.Ut, Kw, nullptr, nullptr, G.Ut, &pos) &&
+           build_grp_factor(ar, L.Lt, Kw, &pos, &L.h_d, G.Lt, nullptr);
+    }
+    if (!ok) return false;
+    for (int b = 0; b < G.ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
+    G.ctr = ar.alloc<int>(32 * 4);
+    reset_grp(L, Kw);
+    return true;
+  }
+  void reset_grp(Lev &L, int Kw) {
+    auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
+    if (!G.ctr) return;
+    const int64_t nn = (int64_t)L.n * Kw;
+    for (int b = 0; b < G.ring; ++b)
+      k_fill<T><<<blocks_for(nn), 256, 0, st>>>((int)nn, Sentinel<T>::value(), G.x[b]);
+    MLDG_CUDA(cudaMemsetAsync(G.ctr, 0, sizeof(int) * 32 * 4, st));
+    G.seq = 0;
+  }
+
   void build_blk_m(DTri<T> &t, int Kw) {
     const int ki = ilog2(Kw), rpw = 32 / Kw;
     const int nl = (int)t.h_lvl.size() - 1;
@@ -2156,6 +2497,7 @@ struct EngineT : Engine {
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    if (L.grp) reset_grp(L, 1);
     const bool keep = t[1] < t[0] || std::getenv("MLDG_DENSE_INV");
     set(keep);  // (rejected matrices stay in the arena until the handle is freed)
     if (std::getenv("MLDG_VERBOSE"))
@@ -2172,6 +2514,7 @@ struct EngineT : Engine {
       marena.release();
       for (auto &L : lv) {
         L.xm = L.ym = L.tym = L.twm = L.tzm = L.bufAm = L.bufBm = nullptr;
+        for (int q = 1; q < 6; ++q) L.g[q] = typename Lev::Grp();
         for (DTri<T> *t : {&L.L, &L.U, &L.Ut, &L.Lt})
           for (int q = 1; q < 6; ++q) {  // [0] (one column) lives in the main arena
             t->blkm[q] = nullptr;
@@ -2202,7 +2545,8 @@ struct EngineT : Engine {
         MLDG_CUDA(cudaMemsetAsync(L.ym, 0, sizeof(T) * n, st));
         MLDG_CUDA(cudaMemsetAsync(L.tym, 0, sizeof(T) * n, st));
         MLDG_CUDA(cudaMemsetAsync(L.twm, 0, sizeof(T) * n, st));
-        if ((L.kind == MLDG_SMOOTHER_BJAC || L.kind == MLDG_SMOOTHER_FBGS) && !L.minv) {
+        if ((L.kind == MLDG_SMOOTHER_BJAC || L.kind == MLDG_SMOOTHER_FBGS) && !L.minv &&
+            (!L.grp || mcap > kGrpCols)) {
           // exchange buffers start as all-sentinel (bufAm stays so after every solve pair)
           L.bufAm = marena.alloc<T>(n);
           L.bufBm = marena.alloc<T>(n);
@@ -2215,6 +2559,10 @@ struct EngineT : Engine {
     const int ki = ilog2(Kw);
     for (auto &L : lv) {
       if ((L.kind != MLDG_SMOOTHER_BJAC && L.kind != MLDG_SMOOTHER_FBGS) || L.minv) continue;
+      if (L.grp && Kw <= kGrpCols) {
+        if (!L.g[ki].ctr && !build_grp(L, Kw, marena)) fail(MLDG_ERR_SIZE, "grouped plan too large for %d columns", Kw);
+        continue;
+      }
       for (DTri<T> *t : {&L.L, &L.U, &L.Ut, &L.Lt}) {
         if (!t->present() && L.kind == MLDG_SMOOTHER_FBGS) continue;
         if (!t->present()) fail(MLDG_ERR_INTERNAL, "multi-RHS solve without a level schedule");
@@ -2345,6 +2693,10 @@ struct EngineT : Engine {
               (int64_t)L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))));
       return;
     }
+    if (L.grp && K <= kGrpCols) {
+      gpair(L, K, trans, x, beta, y);
+      return;
+    }
     if (trans == 'N') {
       trsv_m(L.L, x, nullptr, L.bufAm, L.bufBm, nullptr, T(1), T(0));
       trsv_m(L.U, L.bufAm, L.d, L.bufBm, L.bufAm, y, T(1), beta);
@@ -2365,6 +2717,11 @@ struct EngineT : Engine {
       end((int64_t)L.n * L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))),
           (backward ? L.nnz_u : L.nnz_l) * (int64_t)(sizeof(T) + 4) + 4 * ((int64_t)L.n + 1) +
               (int64_t)L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))));
+      return;
+    }
+    if (L.grp && K <= kGrpCols) {
+      auto &G = L.g[ilog2(K)];
+      gsolve(G, backward ? G.U : G.L, K, backward ? L.nnz_u : L.nnz_l, rhs, out, beta);
       return;
     }
     DTri<T> &t = backward ? L.U : L.L;
@@ -2509,6 +2866,7 @@ struct EngineT : Engine {
     probe_armed = false;
     std::memset(seen, 0, sizeof seen);
     K = Kw;
+    for (auto &L : lv) L.g[ilog2(Kw)].seq = 0;
     Lev &F = lv[0];
     const int64_t n = nk(F.n);
     if (!std::is_same<T, double>::value) {
@@ -2533,6 +2891,7 @@ struct EngineT : Engine {
       vcycle_m(0, trans);
     }
     end_fbgs_m();
+    end_grp(Kw);
     if (!std::is_same<T, double>::value) {
       cur_lev = 0;
       begin(MLDG_KERNEL_VEC);
@@ -2627,6 +2986,7 @@ struct EngineT : Engine {
     cur_lev = 0;
     probe_armed = false;
     std::memset(seen, 0, sizeof seen);
+    for (auto &L : lv) L.g[0].seq = 0;
     Lev &F = lv[0];
     if (!std::is_same<T, double>::value && !kry_io) {
       begin(MLDG_KERNEL_VEC);
@@ -2654,6 +3014,7 @@ struct EngineT : Engine {
       vcycle(0, trans);
     }
     end_fbgs();
+    end_grp(1);
     if (!std::is_same<T, double>::value && !kry_io) {
       cur_lev = 0;
       begin(MLDG_KERNEL_VEC);
@@ -4034,6 +4395,11 @@ static Engine *make_engine(Handle *h) {
   if (const char *ev = std::getenv("MLDG_STG_S")) e->stg_stages = std::max(2, std::min(kStgMaxStages, std::atoi(ev)));
   Arena &ar = h->arena;
   e->lv.resize(h->nlev);
+  // triangular solves: the grouped solve, unless the environment asks for one
+  // of the others
+  bool want_grp = std::getenv("MLDG_NO_GRP") == nullptr;
+  for (const char *v : {"MLDG_ELL1", "MLDG_WIN_ALL", "MLDG_REP_FORCE", "MLDG_REP_MIN", "MLDG_BLK", "MLDG_BLK_FORCE"})
+    want_grp = want_grp && !std::getenv(v);
   for (int l = 0; l < h->nlev; ++l) {
     HostLevel &H = h->host[l];
     auto &L = e->lv[l];
@@ -4071,7 +4437,18 @@ static Engine *make_engine(Handle *h) {
       L.nnz_u = H.U.nnz();
     }
     tick("matrices (A, A^T, P, R upload)");
-    if (H.kind == MLDG_SMOOTHER_BJAC && !std::getenv("MLDG_NO_WIN")) {
+    const bool dense_coarse = H.kind == MLDG_SMOOTHER_BJAC && l == h->nlev - 1 && h->nlev > 1 &&
+                              L.n <= kDenseCoarseRows && !std::getenv("MLDG_NO_DENSE_COARSE");
+    // The grouped solve for every other ILU(0) and GS level, except the large
+    // ILU(0) levels with wide rows (a coarse level's, above eight entries a
+    // row), which the cluster solve runs faster: the fill of a wide row grows
+    // with its square (idim=101 level 1, 129,684 rows of 14 entries: 256 us a
+    // cluster solve, 290 us a grouped one; level 0, 3 entries: 356 -> 167 us).
+    L.grp = want_grp && L.n > 0 && !dense_coarse &&
+            (H.kind == MLDG_SMOOTHER_FBGS ||
+             (H.kind == MLDG_SMOOTHER_BJAC &&
+              (L.n <= 65536 || H.L.nnz() <= 8 * (int64_t)L.n || std::getenv("MLDG_NO_REP"))));
+    if (H.kind == MLDG_SMOOTHER_BJAC && !L.grp && !std::getenv("MLDG_NO_WIN")) {
       const int n = H.A.nr;
       // Single-CTA windows win on small levels; large levels stay on the
       // sync-free solve unless MLDG_WIN_ALL asks for clusters everywhere.
@@ -4164,8 +4541,7 @@ static Engine *make_engine(Handle *h) {
       }
     }
     tick("FBGS factors, ND");
-    if (H.kind == MLDG_SMOOTHER_BJAC && l == h->nlev - 1 && h->nlev > 1 && L.n <= kDenseCoarseRows &&
-        !std::getenv("MLDG_NO_DENSE_COARSE")) {
+    if (dense_coarse) {
       std::vector<double> M, MT;
       dense_ilu_inverse(H.L, H.U, H.d, M, MT);
       std::vector<T> m(M.begin(), M.end()), mt(MT.begin(), MT.end());
@@ -4177,7 +4553,7 @@ static Engine *make_engine(Handle *h) {
     {
       int rep_min = 65536;
       if (const char *ev = std::getenv("MLDG_REP_MIN")) rep_min = std::atoi(ev);
-      if (H.kind == MLDG_SMOOTHER_BJAC && !L.minv && !L.win && L.n > rep_min && !std::getenv("MLDG_NO_REP")) {
+      if (H.kind == MLDG_SMOOTHER_BJAC && !L.minv && !L.win && !L.grp && L.n > rep_min && !std::getenv("MLDG_NO_REP")) {
         int C = 16;
         if (const char *ev = std::getenv("MLDG_REP_C")) C = std::atoi(ev) == 8 ? 8 : 16;
         HostCSR Lt = transpose(H.L), Ut = transpose(H.U);
@@ -4259,7 +4635,12 @@ static Engine *make_engine(Handle *h) {
     MLDG_CUDA(cudaMemset(L.y, 0, sizeof(T) * n));
     MLDG_CUDA(cudaMemset(L.ty, 0, sizeof(T) * n));
     MLDG_CUDA(cudaMemset(L.tw, 0, sizeof(T) * n));
-    if (H.kind == MLDG_SMOOTHER_BJAC || H.kind == MLDG_SMOOTHER_FBGS) {
+    if (L.grp) {
+      L.h_d = dh;
+      L.grp = e->build_grp(L, 1, ar);
+      tick("grouped plans");
+    }
+    if ((H.kind == MLDG_SMOOTHER_BJAC || H.kind == MLDG_SMOOTHER_FBGS) && !L.grp) {
       L.bufA = ar.alloc<T>(n);
       L.bufB = ar.alloc<T>(n);
       k_fill<T><<<64, 256, 0, h->st>>>(n, Sentinel<T>::value(), L.bufA);
@@ -6140,6 +6521,46 @@ extern "C" int mldg_blk_plan_check(const mldg_csr *Tc, int upper, const double *
     if (stats[3]) std::copy(out.begin(), out.end(), t);
   } catch (const mldg::Error &e) {
     return e.code;
+  }
+  return MLDG_SUCCESS;
+}
+
+extern "C" int mldg_grp_plan_check(const mldg_csr *Tc, int upper, const double *scale, const double *rhs, double *t,
+                                   int ncols, long long budget, int row, double growth, int fp32, long long *stats) {
+  if (!Tc || !rhs || !t || !stats || ncols < 1 || ncols > 32 || (ncols & (ncols - 1))) return MLDG_ERR_ARG;
+  try {
+    mldg::HostCSR m = mldg::copy_csr(*Tc, 0, "T", 0);
+    if (m.nr != m.nc || m.nr < 1) return MLDG_ERR_ARG;
+    mldg::TriSchedule s;
+    mldg::build_tri_schedule(m.nr, m.irp.data(), m.ja.data(), m.val.data(), upper != 0, m.nr, &s);
+    std::vector<int> orig, dep;
+    mldg::grp_positions(m.nr, upper != 0, s.prow, s.pja, orig, dep);
+    mldg::TriGroups g;
+    mldg::build_tri_groups(s.lvl_ptr, s.pirp, dep, s.pval, budget > 0 ? budget : mldg::grp_budget(m.nr, ncols),
+                           row > 0 ? row : mldg::kGrpRow, growth > 0 ? growth : mldg::kGrpGrowth, &g);
+    const std::vector<double> r(rhs, rhs + m.nr);
+    std::vector<double> x;
+    auto run = [&](auto tag) {
+      typedef decltype(tag) TT;
+      const int KC = mldg::grp_cols<TT>(ncols);
+      mldg::GrpTasks<TT> tk;
+      const bool ok = mldg::grp_tasks<TT>(
+          g, KC, [&](int c) { return orig[c]; }, [&](int c) { return scale ? scale[orig[c]] : 1.0; }, tk);
+      stats[0] = ok ? mldg::grp_emulate<TT>(g, tk, KC, r, x) : -1;
+      stats[1] = (long long)s.lvl_ptr.size() - 1;
+      stats[2] = (long long)g.gptr.size() - 1;
+      stats[3] = (long long)g.entries;
+    };
+    if (fp32)
+      run(float());
+    else
+      run(double());
+    if (stats[0] < 0) return MLDG_ERR_SIZE;
+    for (int p = 0; p < m.nr; ++p) t[orig[p]] = x[p];
+  } catch (const mldg::Error &e) {
+    return e.code;
+  } catch (const std::exception &) {
+    return MLDG_ERR_ALLOC;
   }
   return MLDG_SUCCESS;
 }
