@@ -15,6 +15,7 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <exception>
 #include <map>
 #include <set>
 #include <cstdarg>
@@ -25,6 +26,7 @@
 #include <mutex>
 #include <string>
 #include <type_traits>
+#include <thread>
 #include <vector>
 
 #include <omp.h>
@@ -456,19 +458,22 @@ struct DBlk {
 };
 
 // Grouped solve: entries of V and W per group, entries of a row, the bound on a
-// row of W, and the widest block of columns.  A group's entries should stream
+// row of W, and the widest block of columns
+// of a narrow level.  A group's entries should stream
 // in about the time of its hand-off, which takes longer the more warps take
 // part: n/5 entries between these limits (solve pair at idim=40, 64,000 rows:
 // 86 us with 50,000 and 100,000, 98 us with 200,000; idim=101, 1,030,301 rows:
-// 333 us with 200,000, 408 us with 100,000).  Blocks above eight columns keep
-// the ELL solve: their gathers move 32 values an entry, so the fill costs more
-// than the hand-offs it saves (32 columns at idim=64: 250 us a solve against 178).
+// 333 us with 200,000, 408 us with 100,000).  Blocks above eight columns
+// move 16 or 32 values an entry, so a group holds fewer entries, and levels of
+// short rows (at most kGrpWide entries) keep the ELL solve (32 columns at
+// idim=64: level 0, 3 entries a row: 250 us a solve, ELL 178; level 1, 14 entries:
+// 304 us, ELL 345).
 constexpr int64_t kGrpBudgetMin = 50000, kGrpBudgetMax = 200000;
 constexpr int kGrpRow = 512;
 constexpr double kGrpGrowth = 64.0;
-constexpr int kGrpCols = 8;
+constexpr int kGrpCols = 8, kGrpWide = 8;
 static int64_t grp_budget(int n, int K) {
-  return K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
+  return K > kGrpCols ? kGrpBudgetMin / 2 : K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
 }
 // columns of one task: a 32-byte sector of a row's K values
 template <typename T>
@@ -477,7 +482,7 @@ constexpr int grp_cols(int K) {
 }
 
 // original row of every position, and the dependencies as positions
-static void grp_positions(int n, bool rev, const std::vector<int> &prow, const std::vector<int> &pja,
+static void grp_positions(int n, bool rev, const std::vector<int> &prow, const std::vector<int> &pja, bool par,
                           std::vector<int> &orig, std::vector<int> &dep) {
   std::vector<int> pos((size_t)n);
   orig.resize((size_t)n);
@@ -486,7 +491,7 @@ static void grp_positions(int n, bool rev, const std::vector<int> &prow, const s
     pos[prow[p]] = p;
     orig[p] = rev ? n - 1 - prow[p] : prow[p];
   }
-#pragma omp parallel for schedule(static, 4096)
+#pragma omp parallel for schedule(static, 4096) if (par)
   for (int64_t k = 0; k < (int64_t)dep.size(); ++k) dep[k] = pos[pja[k]];
 }
 
@@ -501,7 +506,7 @@ struct GrpTasks {
 // wcol(c), wscale(c): index in b and factor of W's column position c; false
 // when the slots outgrow the descriptors
 template <typename T, typename FC, typename FS>
-static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, GrpTasks<T> &out) {
+static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, bool par, GrpTasks<T> &out) {
   const int R = 32 / KC, ng = (int)g.gptr.size() - 1;
   auto len = [&](int p) { return (int64_t)std::max(g.row[p].nv, g.row[p].nw); };
   int64_t at = 0;  // slot groups (one int4 of indices each)
@@ -536,7 +541,7 @@ static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, GrpTasks<T
     }
   out.idx.reset(new int4[(size_t)std::max<int64_t>(at, 1)]);
   out.val.reset(new T[(size_t)std::max<int64_t>(4 * at, 1)]);
-#pragma omp parallel for schedule(static, 64)
+#pragma omp parallel for schedule(static, 64) if (par)
   for (int64_t k = 0; k < (int64_t)out.desc.size(); ++k) {
     const int4 d = out.desc[k];
     const int lt = d.w & 255, rows = d.w >> 8, tpr = 1 << lt;
@@ -986,7 +991,7 @@ struct Engine {
   // Multi-RHS V-cycle on K row-interleaved columns: xin_m -> yout_m (FP64,
   // n0 x K interleaved).  ensure_multi allocates the K-wide buffers (true when
   // they were reallocated, which invalidates captured multi graphs).
-  virtual bool ensure_multi(int K) = 0;
+  virtual bool ensure_multi(int K, char trans) = 0;
   virtual void record_multi(char trans, int K) = 0;
   double *xin_m = nullptr, *yout_m = nullptr, *col_m = nullptr;
   int mcap = 0;
@@ -1194,6 +1199,7 @@ struct EngineT : Engine {
       T *x[4] = {};
       int *ctr = nullptr;  // one ticket counter per buffer
       int ring = 4, seq = 0;
+      bool built(char trans) const { return (trans == 'N' ? L : Ut).n > 0; }
     } g[6];
     // coarsest level: explicit inverse of its ILU(0) factorisation (and its transpose)
     T *minv = nullptr, *minvT = nullptr;
@@ -1676,6 +1682,10 @@ struct EngineT : Engine {
       case 4: f(std::integral_constant<int, 4>()); break;
       default: f(std::integral_constant<int, (int)(32 / sizeof(T))>());
     }
+  }
+  // whether a block of Kw columns takes the grouped solve on a level
+  static bool grp_for(const Lev &L, int Kw) {
+    return L.grp && (Kw <= kGrpCols || L.nnz_l + L.nnz_u > 2 * kGrpWide * (int64_t)L.n);
   }
   void gpair(Lev &L, int Kw, char trans, const T *x, T beta, T *y) {
     auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
@@ -2176,30 +2186,47 @@ struct EngineT : Engine {
   }
   int64_t nk(int n) const { return (int64_t)n * K; }
 
-  // Grouped plan of factor t for Kw columns: rhs_pos (original row -> index of
-  // the right-hand side; null: original order), scale (by original row, or
-  // null); pos_out: original row -> position.
-  bool build_grp_factor(Arena &ar, const DTri<T> &t, int Kw, const std::vector<int> *rhs_pos,
-                        const std::vector<double> *scale, DGrp<T> &g, std::vector<int> *pos_out) {
-    const int n = t.n, KC = grp_cols<T>(Kw);
-    std::vector<int> orig, dep;
-    grp_positions(n, t.rev != 0, t.h_prow, t.h_pja, orig, dep);
-    int64_t budget = grp_budget(n, Kw);
-    if (const char *e = std::getenv("MLDG_GRP_B")) budget = std::max(1, std::atoi(e));
+  // The host side of a factor's grouped plan for Kw columns; W reads the
+  // solution of `src` (null: a vector in original order) scaled by `scale` (by
+  // original row, or null).  par: with OpenMP inside.
+  struct GrpHost {
+    const DTri<T> *t = nullptr, *src = nullptr;
+    const std::vector<double> *scale = nullptr;
+    DGrp<T> *dst = nullptr;
+    bool ok = false;
+    std::exception_ptr error;
+    std::vector<int> orig;
     TriGroups pl;
-    build_tri_groups(t.h_lvl, t.h_pirp, dep, t.h_pval, budget, kGrpRow, kGrpGrowth, &pl);
     GrpTasks<T> tk;
-    if (!grp_tasks<T>(
-            pl, KC, [&](int c) { return rhs_pos ? (*rhs_pos)[orig[c]] : orig[c]; },
-            [&](int c) { return scale ? (*scale)[orig[c]] : 1.0; }, tk))
-      return false;
+    void build(int Kw, bool par) {
+      const int n = t->n;
+      std::vector<int> dep, at;
+      grp_positions(n, t->rev != 0, t->h_prow, t->h_pja, par, orig, dep);
+      if (src) {
+        at.resize((size_t)n);
+        for (int p = 0; p < n; ++p) at[src->rev ? n - 1 - src->h_prow[p] : src->h_prow[p]] = p;
+      }
+      int64_t budget = grp_budget(n, Kw);
+      if (const char *e = std::getenv("MLDG_GRP_B")) budget = std::max(1, std::atoi(e));
+      build_tri_groups(t->h_lvl, t->h_pirp, dep, t->h_pval, budget, kGrpRow, kGrpGrowth, par, &pl);
+      ok = grp_tasks<T>(
+          pl, grp_cols<T>(Kw), [&](int c) { return src ? at[orig[c]] : orig[c]; },
+          [&](int c) { return scale ? (*scale)[orig[c]] : 1.0; }, par, tk);
+    }
+  };
+  // its device side; the host's copies are released
+  void upload_grp(Arena &ar, GrpHost &hp, int Kw) {
+    const DTri<T> &t = *hp.t;
+    DGrp<T> &g = *hp.dst;
+    GrpTasks<T> &tk = hp.tk;
+    const int n = t.n, KC = grp_cols<T>(Kw);
     g.n = n;
     g.slots = tk.slots;
     g.m.ntask = (int)tk.desc.size();
     g.m.desc = ar.upload(tk.desc);
     g.m.idx = ar.upload(tk.idx.get(), (size_t)tk.slots / 4);
     g.m.val = ar.upload(tk.val.get(), (size_t)tk.slots);
-    g.orig = ar.upload(orig);
+    g.orig = ar.upload(hp.orig);
     // warps in flight: eight groups' tasks, so that a group's tasks have their
     // entries and older values loaded when the group before it is finished
     // (idim=101 level 0: 822 us for four solves with four groups, 680 with eight)
@@ -2207,38 +2234,68 @@ struct EngineT : Engine {
     grp_dispatch(Kw, [&](auto kc) {
       MLDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trsv_grp<T, decltype(kc)::value>, 256, 0));
     });
-    const int ng = (int)pl.gptr.size() - 1;
+    const int ng = (int)hp.pl.gptr.size() - 1;
     const int64_t ntask = (int64_t)g.m.ntask * (Kw / KC), per = (ntask + ng - 1) / ng;
-    const int64_t warps = std::max<int64_t>(32, std::min<int64_t>(8 * per, ntask));
+    const int64_t warps = std::max<int64_t>(32, std::min<int64_t>((Kw > kGrpCols ? 4 : 8) * per, ntask));
     g.grid = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, (int64_t)std::max(nb, 1) * nsm));
     if (std::getenv("MLDG_VERBOSE"))
       std::fprintf(stderr, "mldg: grp K=%d n=%d levels=%d groups=%d entries %lld slots %lld tasks %d grid %d occ %d\n", Kw, n,
-                   t.nlevels, ng, (long long)pl.entries, (long long)g.slots, g.m.ntask, g.grid, nb);
-    if (pos_out) {
-      pos_out->resize((size_t)n);
-      for (int p = 0; p < n; ++p) (*pos_out)[orig[p]] = p;
-    }
-    return true;
+                   t.nlevels, ng, (long long)hp.pl.entries, (long long)g.slots, g.m.ntask, g.grid, nb);
+    hp = GrpHost();
   }
-  // the grouped plans and work vectors of a level for Kw columns
-  bool build_grp(Lev &L, int Kw, Arena &ar) {
+  // The grouped plans (of trans 'N' or 'T', or of both: 0) and work vectors of a
+  // level for Kw columns.  A small
+  // level's factors are planned by a thread each (their levels are too narrow to
+  // share), a large one's in turn by all threads.
+  bool build_grp(Lev &L, int Kw, char trans, Arena &ar) {
     auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
-    bool ok;
+    std::vector<GrpHost> hp;
+    auto add = [&](const DTri<T> &t, const DTri<T> *src, const std::vector<double> *scale, DGrp<T> &dst) {
+      hp.emplace_back();
+      hp.back().t = &t;
+      hp.back().src = src;
+      hp.back().scale = scale;
+      hp.back().dst = &dst;
+    };
     if (L.kind == MLDG_SMOOTHER_FBGS) {
       G.ring = 2;
-      ok = build_grp_factor(ar, L.L, Kw, nullptr, &L.h_d, G.L, nullptr) &&
-           build_grp_factor(ar, L.U, Kw, nullptr, &L.h_d, G.U, nullptr);
+      add(L.L, nullptr, &L.h_d, G.L);
+      add(L.U, nullptr, &L.h_d, G.U);
     } else {
-      std::vector<int> pos;
-      ok = build_grp_factor(ar, L.L, Kw, nullptr, nullptr, G.L, &pos) &&
-           build_grp_factor(ar, L.U, Kw, &pos, &L.h_d, G.U, nullptr) &&
-           build_grp_factor(ar, L.Ut, Kw, nullptr, nullptr, G.Ut, &pos) &&
-           build_grp_factor(ar, L.Lt, Kw, &pos, &L.h_d, G.Lt, nullptr);
+      if (trans != 'T') {
+        add(L.L, nullptr, nullptr, G.L);
+        add(L.U, &L.L, &L.h_d, G.U);
+      }
+      if (trans != 'N') {
+        add(L.Ut, nullptr, nullptr, G.Ut);
+        add(L.Lt, &L.Ut, &L.h_d, G.Lt);
+      }
     }
-    if (!ok) return false;
-    for (int b = 0; b < G.ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
-    G.ctr = ar.alloc<int>(32 * 4);
-    reset_grp(L, Kw);
+    if (L.n <= 262144) {
+      std::vector<std::thread> th;
+      auto run = [Kw](GrpHost *p) {
+        try {
+          p->build(Kw, false);
+        } catch (...) {
+          p->error = std::current_exception();
+        }
+      };
+      for (size_t k = 1; k < hp.size(); ++k) th.emplace_back(run, &hp[k]);
+      run(&hp[0]);
+      for (auto &t : th) t.join();
+    } else {
+      for (auto &p : hp) p.build(Kw, true);
+    }
+    for (auto &p : hp)
+      if (p.error) std::rethrow_exception(p.error);
+    for (auto &p : hp)
+      if (!p.ok) return false;
+    for (auto &p : hp) upload_grp(ar, p, Kw);
+    if (!G.ctr) {
+      for (int b = 0; b < G.ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
+      G.ctr = ar.alloc<int>(32 * 4);
+      reset_grp(L, Kw);
+    }
     return true;
   }
   void reset_grp(Lev &L, int Kw) {
@@ -2463,7 +2520,6 @@ struct EngineT : Engine {
     }
     for (DTri<T> *f : {&L.L, &L.U}) f->ell[ki] = typename DTri<T>::Ell();
     tmp.release();
-    if (!ok) return false;
     // keep the dense form only if it is faster
     auto op = [&]() {
       if (gs) {
@@ -2508,7 +2564,7 @@ struct EngineT : Engine {
     impl_bytes = 0;
     return keep;
   }
-  bool ensure_multi(int Kw) override {
+  bool ensure_multi(int Kw, char trans) override {
     bool grown = false;
     if (Kw > mcap) {
       marena.release();
@@ -2546,7 +2602,7 @@ struct EngineT : Engine {
         MLDG_CUDA(cudaMemsetAsync(L.tym, 0, sizeof(T) * n, st));
         MLDG_CUDA(cudaMemsetAsync(L.twm, 0, sizeof(T) * n, st));
         if ((L.kind == MLDG_SMOOTHER_BJAC || L.kind == MLDG_SMOOTHER_FBGS) && !L.minv &&
-            (!L.grp || mcap > kGrpCols)) {
+            !grp_for(L, mcap)) {
           // exchange buffers start as all-sentinel (bufAm stays so after every solve pair)
           L.bufAm = marena.alloc<T>(n);
           L.bufBm = marena.alloc<T>(n);
@@ -2559,8 +2615,8 @@ struct EngineT : Engine {
     const int ki = ilog2(Kw);
     for (auto &L : lv) {
       if ((L.kind != MLDG_SMOOTHER_BJAC && L.kind != MLDG_SMOOTHER_FBGS) || L.minv) continue;
-      if (L.grp && Kw <= kGrpCols) {
-        if (!L.g[ki].ctr && !build_grp(L, Kw, marena)) fail(MLDG_ERR_SIZE, "grouped plan too large for %d columns", Kw);
+      if (grp_for(L, Kw)) {
+        if (!L.g[ki].built(trans) && !build_grp(L, Kw, trans, marena)) fail(MLDG_ERR_SIZE, "grouped plan too large for %d columns", Kw);
         continue;
       }
       for (DTri<T> *t : {&L.L, &L.U, &L.Ut, &L.Lt}) {
@@ -2576,23 +2632,36 @@ struct EngineT : Engine {
     return grown;
   }
 
-  void spmm(const DCSR<T> &A, const T *v, T a1, const T *b, T a0, T *out, T a2) {
-    const int g = blocks_for(nk(A.nr));
-    begin(MLDG_KERNEL_SPMV);
+  // K columns, and whether the lanes a row leaves share its entries: from 16
+  // entries a row (restriction to 910 rows of 187 entries, 32 columns: 62 us
+  // unsplit)
+  template <typename F>
+  static void spmm_dispatch(int K, int64_t nnz, int nr, F &&f) {
     kdispatch(K, [&](auto kc) {
-      constexpr int KK = decltype(kc)::value;
-      k_spmm<T, KK><<<g, 256, 0, st>>>(A.nr, A.irp, A.ja, A.val, v, a1, b, a0, out, a2);
+      constexpr int SP = kSpmmSplit<T, decltype(kc)::value>;
+      if (SP > 1 && nnz >= 16 * (int64_t)nr)
+        f(kc, std::integral_constant<int, SP>());
+      else
+        f(kc, std::integral_constant<int, 1>());
+    });
+  }
+  void spmm(const DCSR<T> &A, const T *v, T a1, const T *b, T a0, T *out, T a2) {
+    begin(MLDG_KERNEL_SPMV);
+    spmm_dispatch(K, A.nnz, A.nr, [&](auto kc, auto sp) {
+      constexpr int KK = decltype(kc)::value, SP = decltype(sp)::value;
+      k_spmm<T, KK, SP><<<blocks_for((int64_t)A.nr * (KK / kVecCols<T, KK>) * SP), 256, 0, st>>>(
+          A.nr, A.irp, A.ja, A.val, v, a1, b, a0, out, a2);
     });
     end(A.nnz * (int64_t)(sizeof(T) + 4) + 4 * ((int64_t)A.nr + 1) + nk(A.nc) * (int64_t)sizeof(T) +
         nk(A.nr) * (int64_t)sizeof(T) * (1 + (b ? 1 : 0) + (a2 != T(0) ? 1 : 0)));
   }
   void jacobi_m(const DCSR<T> &ND, const T *d, const T *x, const T *ty, int first, T omega, T alpha, T beta,
                 T *out) {
-    const int g = blocks_for(nk(ND.nr));
     begin(MLDG_KERNEL_JACOBI);
-    kdispatch(K, [&](auto kc) {
-      constexpr int KK = decltype(kc)::value;
-      k_jacobi_m<T, KK><<<g, 256, 0, st>>>(ND.nr, ND.irp, ND.ja, ND.val, d, x, ty, first, omega, alpha, beta, out);
+    spmm_dispatch(K, ND.nnz, ND.nr, [&](auto kc, auto sp) {
+      constexpr int KK = decltype(kc)::value, SP = decltype(sp)::value;
+      k_jacobi_m<T, KK, SP><<<blocks_for((int64_t)ND.nr * (KK / kVecCols<T, KK>) * SP), 256, 0, st>>>(
+          ND.nr, ND.irp, ND.ja, ND.val, d, x, ty, first, omega, alpha, beta, out);
     });
     end(ND.nnz * (int64_t)(sizeof(T) + 4) + 4 * ((int64_t)ND.nr + 1) + (int64_t)ND.nr * sizeof(T) +
         nk(ND.nr) * (int64_t)sizeof(T) * (2 + (first ? 0 : 1) + (beta != T(0) ? 1 : 0)));
@@ -2680,20 +2749,29 @@ struct EngineT : Engine {
       });
     }
   }
+  // out = M x + beta*out, M dense n x n (a level's explicit inverse)
+  void gemm_m(int n, const T *M, const T *x, T beta, T *out) {
+    kdispatch(K, [&](auto kc) {
+      constexpr int KK = decltype(kc)::value;
+      if constexpr (KK <= 8)
+        k_gemm_m_rows<T, KK><<<std::max(1, std::min((n * KK + 127) / 128, nsm * 16)), 128, 0, st>>>(n, M, x, T(1), beta,
+                                                                                                 out);
+      else
+        k_gemm_m_cols<T, KK><<<std::max(1, std::min((n * KK + 127) / 128, nsm * 8)), 256, 0, st>>>(n, M, x, T(1), beta,
+                                                                                                out);
+    });
+  }
   void ilu_apply_m(Lev &L, char trans, const T *x, T beta, T *y) {
     if (L.minv) {
       const T *M = (trans == 'N') ? L.minv : L.minvT;
       begin(MLDG_KERNEL_VEC);
-      kdispatch(K, [&](auto kc) {
-        constexpr int KK = decltype(kc)::value;
-        k_gemm_m<T, KK><<<blocks_for(nk(L.n)), 256, 0, st>>>(L.n, M, x, T(1), beta, y);
-      });
+      gemm_m(L.n, M, x, beta, y);
       end((int64_t)L.n * L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))),
           (L.nnz_l + L.nnz_u) * (int64_t)(sizeof(T) + 4) + 8 * ((int64_t)L.n + 1) +
               (int64_t)L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))));
       return;
     }
-    if (L.grp && K <= kGrpCols) {
+    if (grp_for(L, K)) {
       gpair(L, K, trans, x, beta, y);
       return;
     }
@@ -2710,16 +2788,13 @@ struct EngineT : Engine {
     if (L.gsF) {
       const T *M = backward ? L.gsB : L.gsF;
       begin(MLDG_KERNEL_VEC);
-      kdispatch(K, [&](auto kc) {
-        constexpr int KK = decltype(kc)::value;
-        k_gemm_m<T, KK><<<blocks_for(nk(L.n)), 256, 0, st>>>(L.n, M, rhs, T(1), beta, out);
-      });
+      gemm_m(L.n, M, rhs, beta, out);
       end((int64_t)L.n * L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))),
           (backward ? L.nnz_u : L.nnz_l) * (int64_t)(sizeof(T) + 4) + 4 * ((int64_t)L.n + 1) +
               (int64_t)L.n * sizeof(T) + nk(L.n) * (int64_t)sizeof(T) * (2 + (beta != T(0))));
       return;
     }
-    if (L.grp && K <= kGrpCols) {
+    if (grp_for(L, K)) {
       auto &G = L.g[ilog2(K)];
       gsolve(G, backward ? G.U : G.L, K, backward ? L.nnz_u : L.nnz_l, rhs, out, beta);
       return;
@@ -4637,7 +4712,7 @@ static Engine *make_engine(Handle *h) {
     MLDG_CUDA(cudaMemset(L.tw, 0, sizeof(T) * n));
     if (L.grp) {
       L.h_d = dh;
-      L.grp = e->build_grp(L, 1, ar);
+      L.grp = e->build_grp(L, 1, 0, ar);
       tick("grouped plans");
     }
     if ((H.kind == MLDG_SMOOTHER_BJAC || H.kind == MLDG_SMOOTHER_FBGS) && !L.grp) {
@@ -4957,15 +5032,15 @@ static int width_for(int k) {
   while (K < k) K *= 2;
   return K;
 }
-static void prepare_multi(Handle *h, int K) {
-  if (h->eng->ensure_multi(K)) drop_multi_graphs(h);
+static void prepare_multi(Handle *h, int K, char trans) {
+  if (h->eng->ensure_multi(K, trans)) drop_multi_graphs(h);
 }
 
 // nrhs > 1: blocks of up to 32 columns through the K-wide V-cycle
 static void apply_multi(Handle *h, const double *x, double *y, char trans, int nrhs, int ld, int mem) {
   for (int c0 = 0; c0 < nrhs; c0 += 32) {
     const int k = std::min(32, nrhs - c0), K = width_for(k);
-    prepare_multi(h, K);
+    prepare_multi(h, K, trans);
     load_block(h, x + (size_t)c0 * ld, ld, k, K, mem, h->eng->xin_m);
     run_vcycle_multi(h, trans, K);
     store_block(h, h->eng->yout_m, k, K, mem, y + (size_t)c0 * ld, ld);
@@ -5367,10 +5442,10 @@ static void scal_m(Handle *h, int K, int what) {
 }
 static void spmm64(Handle *h, int K, const DCSR<double> &A, const double *v, double a1, const double *b, double a0,
                    double *out) {
-  const int64_t thr = (int64_t)A.nr * K;
+  const int64_t thr = (int64_t)A.nr * K / 2;
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>((thr + 255) / 256, (int64_t)h->nsm * 16));
   kdispatch(K, [&](auto kc) {
-    k_spmm<double, decltype(kc)::value><<<g, 256, 0, h->st>>>(A.nr, A.irp, A.ja, A.val, v, a1, b, a0, out, 0.0);
+    k_spmm<double, decltype(kc)::value, 1><<<g, 256, 0, h->st>>>(A.nr, A.irp, A.ja, A.val, v, a1, b, a0, out, 0.0);
   });
   h->last_launches++;
 }
@@ -5410,7 +5485,7 @@ static void krylov_multi(Handle *h, int method, const mldg_csr *Acsr, int nrhs, 
   MLDG_CUDA(cudaEventRecord(h->ev0, h->st));
   for (int c0 = 0; c0 < nrhs; c0 += 32) {
     const int k = std::min(32, nrhs - c0), K = width_for(k);
-    prepare_multi(h, K);
+    prepare_multi(h, K, 'N');
     ensure_krylov_m(h, K);
     Engine &e = *h->eng;
     double *r = e.xin_m, *z = e.yout_m, *d = h->kd_m, *q = h->kq_m, *xx = h->kx_m, *bb = h->kb_m;
@@ -6061,7 +6136,7 @@ static void profile_run(Handle &h, char trans, int nrhs, int max, mldg_kernel_st
   mldg::check_trans(&h, trans);
   if (nrhs < 1 || nrhs > 32) mldg::fail(MLDG_ERR_ARG, "profile width must be 1..32");
   const int K = nrhs > 1 ? mldg::width_for(nrhs) : 1;
-  if (K > 1) mldg::prepare_multi(&h, K);
+  if (K > 1) mldg::prepare_multi(&h, K, trans);
   std::vector<mldg::Engine::Prof> prof;
   h.eng->prof = &prof;
   const int pk = h.eng->probe_kind;
@@ -6534,10 +6609,10 @@ extern "C" int mldg_grp_plan_check(const mldg_csr *Tc, int upper, const double *
     mldg::TriSchedule s;
     mldg::build_tri_schedule(m.nr, m.irp.data(), m.ja.data(), m.val.data(), upper != 0, m.nr, &s);
     std::vector<int> orig, dep;
-    mldg::grp_positions(m.nr, upper != 0, s.prow, s.pja, orig, dep);
+    mldg::grp_positions(m.nr, upper != 0, s.prow, s.pja, true, orig, dep);
     mldg::TriGroups g;
     mldg::build_tri_groups(s.lvl_ptr, s.pirp, dep, s.pval, budget > 0 ? budget : mldg::grp_budget(m.nr, ncols),
-                           row > 0 ? row : mldg::kGrpRow, growth > 0 ? growth : mldg::kGrpGrowth, &g);
+                           row > 0 ? row : mldg::kGrpRow, growth > 0 ? growth : mldg::kGrpGrowth, true, &g);
     const std::vector<double> r(rhs, rhs + m.nr);
     std::vector<double> x;
     auto run = [&](auto tag) {
@@ -6545,7 +6620,7 @@ extern "C" int mldg_grp_plan_check(const mldg_csr *Tc, int upper, const double *
       const int KC = mldg::grp_cols<TT>(ncols);
       mldg::GrpTasks<TT> tk;
       const bool ok = mldg::grp_tasks<TT>(
-          g, KC, [&](int c) { return orig[c]; }, [&](int c) { return scale ? scale[orig[c]] : 1.0; }, tk);
+          g, KC, [&](int c) { return orig[c]; }, [&](int c) { return scale ? scale[orig[c]] : 1.0; }, true, tk);
       stats[0] = ok ? mldg::grp_emulate<TT>(g, tk, KC, r, x) : -1;
       stats[1] = (long long)s.lvl_ptr.size() - 1;
       stats[2] = (long long)g.gptr.size() - 1;

@@ -10,22 +10,82 @@
 
 namespace mldg {
 
-// out[i,c] = a0*b[i,c] + a1*(A v)[i,c] + a2*out[i,c]
+// Columns a thread handles: a 16-byte vector of a row's K values, so that a
+// row's entries and indices are loaded once for all of them.
 template <typename T, int K>
+constexpr int kVecCols = K * sizeof(T) >= 16 ? 16 / (int)sizeof(T) : K;
+template <typename T, int C>
+struct alignas(C * sizeof(T)) VecCols {
+  T e[C];
+};
+
+// Sum over a row's entries k0 <= k < e of val[k] times the C columns of v's row
+// ja[k], four entries' loads in flight.  SP lanes share the row's entries (four
+// at a time each, a butterfly adds them): 1 for short rows, the lanes a warp
+// has left for long ones, whose chain of loads would bound the kernel.
+template <typename T, int K, int C, int SP, typename F>
+__device__ __forceinline__ VecCols<T, C> spmm_row(int k0, int e, int sp, const int *__restrict__ ja,
+                                                  const T *__restrict__ val, const T *__restrict__ v, int c0, F f) {
+  VecCols<T, C> s;
+#pragma unroll
+  for (int q = 0; q < C; ++q) s.e[q] = T(0);
+  for (int k = k0 + 4 * sp; k < e; k += 4 * SP) {
+    T a[4];
+    VecCols<T, C> x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int kk = min(k + u, e - 1);
+      const int j = __ldg(ja + kk);
+      a[u] = __ldg(val + kk);
+      x[u] = *reinterpret_cast<const VecCols<T, C> *>(v + (size_t)j * K + c0);
+#pragma unroll
+      for (int q = 0; q < C; ++q) x[u].e[q] = f(x[u].e[q], j);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (k + u < e)
+#pragma unroll
+        for (int q = 0; q < C; ++q) s.e[q] = fma(a[u], x[u].e[q], s.e[q]);
+  }
+  if (SP > 1) {
+#pragma unroll
+    for (int o = 16; o >= K / C; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < C; ++q) s.e[q] += __shfl_xor_sync(0xffffffffu, s.e[q], o);
+  }
+  return s;
+}
+// lanes of a warp that a row leaves unused: the entry split of long rows
+template <typename T, int K>
+constexpr int kSpmmSplit = 32 / (K / kVecCols<T, K>);
+
+// out[i,c] = a0*b[i,c] + a1*(A v)[i,c] + a2*out[i,c].  A thread per (row, 16
+// bytes of columns, entry split); bound by HBM on the large levels (level 0 at
+// idim=64, 32 FP32 columns: 41 us a residual, 72 us with a column a thread) and
+// by the rows' chains of loads on the small ones.
+template <typename T, int K, int SP>
 __global__ void __launch_bounds__(256) k_spmm(int nr, const int *__restrict__ irp, const int *__restrict__ ja,
                                               const T *__restrict__ val, const T *__restrict__ v, T a1,
                                               const T *__restrict__ b, T a0, T *out, T a2) {
-  const long long total = (long long)nr * K;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int row = (int)(t / K), c = (int)(t % K);
-    T s = T(0);
-    const int e = irp[row + 1];
-    for (int k = irp[row]; k < e; ++k) s = fma(val[k], __ldg(v + (size_t)ja[k] * K + c), s);
-    T r = a1 * s;
-    if (b) r = fma(a0, b[t], r);
-    if (a2 != T(0)) r = fma(a2, out[t], r);
-    out[t] = r;
+  constexpr int C = kVecCols<T, K>, G = K / C;
+  const long long total = (long long)nr * G * SP, stride = (long long)gridDim.x * blockDim.x;
+  // (SP > 1: a warp is one row, so all its lanes take part in the sums)
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += stride) {
+    const int row = (int)(t / (G * SP)), c0 = (int)(t % G) * C, sp = (int)(t / G) % SP;
+    VecCols<T, C> s = spmm_row<T, K, C, SP>(irp[row], irp[row + 1], sp, ja, val, v, c0, [](T x, int) { return x; });
+    if (sp) continue;
+    const size_t o = (size_t)row * K + c0;
+    VecCols<T, C> bv, ov;
+    if (b) bv = *reinterpret_cast<const VecCols<T, C> *>(b + o);
+    if (a2 != T(0)) ov = *reinterpret_cast<const VecCols<T, C> *>(out + o);
+#pragma unroll
+    for (int q = 0; q < C; ++q) {
+      T r = a1 * s.e[q];
+      if (b) r = fma(a0, bv.e[q], r);
+      if (a2 != T(0)) r = fma(a2, ov.e[q], r);
+      s.e[q] = r;
+    }
+    *reinterpret_cast<VecCols<T, C> *>(out + o) = s;
   }
 }
 
@@ -45,30 +105,31 @@ __global__ void __launch_bounds__(256) k_spmm_h(int nr, const int *__restrict__ 
   }
 }
 
-// multi-RHS point-Jacobi sweep (same algebra as k_jacobi)
-template <typename T, int K>
+// multi-RHS point-Jacobi sweep (same algebra as k_jacobi, threads as in k_spmm)
+template <typename T, int K, int SP>
 __global__ void __launch_bounds__(256) k_jacobi_m(int nr, const int *__restrict__ irp, const int *__restrict__ ja,
                                                   const T *__restrict__ val, const T *__restrict__ d,
                                                   const T *__restrict__ x, const T *__restrict__ ty, int first,
                                                   T omega, T alpha, T beta, T *out) {
-  const long long total = (long long)nr * K;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int row = (int)(t / K), c = (int)(t % K);
-    T s = T(0);
-    const int e = irp[row + 1];
-    if (first == 2) {
-      for (int k = irp[row]; k < e; ++k) s = fma(val[k], omega * __ldg(x + (size_t)ja[k] * K + c), s);
-    } else if (first) {
-      for (int k = irp[row]; k < e; ++k) {
-        const int j = ja[k];
-        s = fma(val[k], omega * (__ldg(d + j) * __ldg(x + (size_t)j * K + c)), s);
-      }
-    } else {
-      for (int k = irp[row]; k < e; ++k) s = fma(val[k], __ldg(ty + (size_t)ja[k] * K + c), s);
-    }
-    out[t] = jac_row(d[row], x[t], s, (!first && omega != T(1)) ? ty[t] : T(0), first != 0, omega, alpha, beta,
-                     beta != T(0) ? out[t] : T(0));
+  constexpr int C = kVecCols<T, K>, G = K / C;
+  const long long total = (long long)nr * G * SP, stride = (long long)gridDim.x * blockDim.x;
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += stride) {
+    const int row = (int)(t / (G * SP)), c0 = (int)(t % G) * C, sp = (int)(t / G) % SP;
+    const int k0 = irp[row], e = irp[row + 1];
+    VecCols<T, C> s;
+    if (first == 2)
+      s = spmm_row<T, K, C, SP>(k0, e, sp, ja, val, x, c0, [&](T xj, int) { return omega * xj; });
+    else if (first)
+      s = spmm_row<T, K, C, SP>(k0, e, sp, ja, val, x, c0, [&](T xj, int j) { return omega * (__ldg(d + j) * xj); });
+    else
+      s = spmm_row<T, K, C, SP>(k0, e, sp, ja, val, ty, c0, [](T xj, int) { return xj; });
+    if (sp) continue;
+    const size_t o = (size_t)row * K + c0;
+#pragma unroll
+    for (int q = 0; q < C; ++q)
+      s.e[q] = jac_row(d[row], x[o + q], s.e[q], (!first && omega != T(1)) ? ty[o + q] : T(0), first != 0, omega, alpha,
+                       beta, beta != T(0) ? out[o + q] : T(0));
+    *reinterpret_cast<VecCols<T, C> *>(out + o) = s;
   }
 }
 
@@ -84,20 +145,106 @@ __global__ void k_diag_m(int n, const T *__restrict__ d, const T *__restrict__ x
   }
 }
 
-// dense coarsest solve for K right-hand sides: out = alpha*M x + beta*out
+// Dense solve for K right-hand sides (a level's explicit inverse): out =
+// alpha*M x + beta*out, M row-major n x n, x and out K-interleaved in 16-byte
+// aligned buffers.
+//
+// K <= 8: a warp forms 32/K rows, its lanes across the columns of M, so that M
+// is read once, coalesced, against K contiguous values of x; each lane holds
+// 32 partial sums, which 31 shuffles turn into one output each.  Wider blocks:
+// a lane per column of x and four rows a lane, blocks of eight warps, which split
+// the columns of M; x is then the coalesced operand and M's entries are
+// broadcast.  (One thread per output, walking its whole row, took 43-99 us for
+// n = 910, K = 32 in FP32 and 1.1 ms for n = 10,978, K = 8 in FP64: a serial
+// chain of n loads.)
 template <typename T, int K>
-__global__ void __launch_bounds__(256) k_gemm_m(int n, const T *__restrict__ M, const T *__restrict__ x, T alpha,
-                                                T beta, T *out) {
-  const long long total = (long long)n * K;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(t / K), c = (int)(t % K);
-    const T *row = M + (size_t)i * n;
-    T s = T(0);
-    for (int j = 0; j < n; ++j) s = fma(__ldg(row + j), __ldg(x + (size_t)j * K + c), s);
-    T r = alpha * s;
-    if (beta != T(0)) r = fma(beta, out[t], r);
-    out[t] = r;
+__device__ __forceinline__ void load_cols(const T *p, T (&v)[K]) {
+  struct alignas(K * sizeof(T) >= 16 ? 16 : K * sizeof(T)) Vec {
+    T e[K * sizeof(T) >= 16 ? 16 / sizeof(T) : K];
+  };
+  constexpr int N = (int)(sizeof(Vec) / sizeof(T));
+#pragma unroll
+  for (int q = 0; q < K / N; ++q) {
+    const Vec w = reinterpret_cast<const Vec *>(p)[q];
+#pragma unroll
+    for (int e = 0; e < N; ++e) v[q * N + e] = w.e[e];
+  }
+}
+template <typename T, int K>
+__global__ void __launch_bounds__(128) k_gemm_m_rows(int n, const T *__restrict__ M, const T *__restrict__ x, T alpha,
+                                                     T beta, T *out) {
+  constexpr int RW = 32 / K;
+  const int lane = threadIdx.x & 31;
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int nwarps = (int)((gridDim.x * blockDim.x) >> 5);
+  for (int i0 = warp * RW; i0 < n; i0 += nwarps * RW) {
+    T acc[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) acc[q] = T(0);
+#pragma unroll 2
+    for (int j = lane; j < n; j += 32) {
+      T xv[K], m[RW];
+      load_cols<T, K>(x + (size_t)j * K, xv);
+#pragma unroll
+      for (int r = 0; r < RW; ++r) m[r] = __ldg(M + (size_t)min(i0 + r, n - 1) * n + j);
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+#pragma unroll
+        for (int c = 0; c < K; ++c) acc[r * K + c] = fma(m[r], xv[c], acc[r * K + c]);
+    }
+    // lane l ends with the sum of acc[l]: output (i0 + l / K, l % K)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int q = 0; q < o; ++q) {
+        const bool up = lane & o;
+        const T send = up ? acc[q] : acc[q + o], keep = up ? acc[q + o] : acc[q];
+        acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    if (i0 + lane / K < n) {
+      const size_t t = (size_t)i0 * K + lane;
+      T r = alpha * acc[0];
+      if (beta != T(0)) r = fma(beta, out[t], r);
+      out[t] = r;
+    }
+  }
+}
+template <typename T, int K>
+__global__ void __launch_bounds__(256) k_gemm_m_cols(int n, const T *__restrict__ M, const T *__restrict__ x, T alpha,
+                                                     T beta, T *out) {
+  constexpr int RG = 32 / K, RW = 4, ROWS = RG * RW;  // row groups of a warp, rows of a lane, rows of a block
+  __shared__ T part[8][ROWS * K];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = lane % K, rg = lane / K;
+  const int j0 = (int)((long long)n * w / 8), j1 = (int)((long long)n * (w + 1) / 8);
+  for (int i0 = blockIdx.x * ROWS; i0 < n; i0 += gridDim.x * ROWS) {
+    T acc[RW];
+    const T *row[RW];
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+      acc[r] = T(0);
+      row[r] = M + (size_t)min(i0 + rg * RW + r, n - 1) * n;
+    }
+#pragma unroll 8
+    for (int j = j0; j < j1; ++j) {
+      const T xv = __ldg(x + (size_t)j * K + c);
+#pragma unroll
+      for (int r = 0; r < RW; ++r) acc[r] = fma(__ldg(row[r] + j), xv, acc[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < RW; ++r) part[w][(rg * RW + r) * K + c] = acc[r];
+    __syncthreads();
+    for (int q = threadIdx.x; q < ROWS * K; q += 256) {
+      if (i0 + q / K < n) {
+        T s = part[0][q];
+#pragma unroll
+        for (int v = 1; v < 8; ++v) s += part[v][q];
+        const size_t t = (size_t)i0 * K + q;
+        T r = alpha * s;
+        if (beta != T(0)) r = fma(beta, out[t], r);
+        out[t] = r;
+      }
+    }
+    __syncthreads();
   }
 }
 

@@ -1,5 +1,5 @@
 // mldg_trigrp.cpp -- see mldg_trigrp.h.  The rows of one level depend only on
-// earlier levels, so a level's rows are formed in parallel; each row is formed
+// earlier levels, so a level's rows may be formed in parallel; each row is formed
 // by one thread in stored order, so the plan does not depend on the number of
 // threads.
 #include "mldg_trigrp.h"
@@ -86,12 +86,13 @@ struct Worker {
 }  // namespace
 
 void build_tri_groups(const std::vector<int> &lvl_ptr, const std::vector<int> &irp, const std::vector<int> &dep,
-                      const std::vector<double> &val, int64_t budget, int row, double growth, TriGroups *out) {
+                      const std::vector<double> &val, int64_t budget, int row, double growth, bool par,
+                      TriGroups *out) {
   const int nl = (int)lvl_ptr.size() - 1, n = nl > 0 ? lvl_ptr[nl] : 0;
   out->gptr.assign(1, 0);
   out->row.resize((size_t)n);
   std::vector<GroupRow> &rows = out->row;
-  std::vector<Worker> workers((size_t)omp_get_max_threads());
+  std::vector<Worker> workers(par ? (size_t)omp_get_max_threads() : 1);
   out->store.resize(workers.size());
   for (size_t t = 0; t < workers.size(); ++t) workers[t].blocks = &out->store[t];
   // the rows of level L in a group that starts at position g0: entries, or -1
@@ -100,9 +101,9 @@ void build_tri_groups(const std::vector<int> &lvl_ptr, const std::vector<int> &i
     int64_t tot = 0;
     int wild = 0;
     const int p0 = lvl_ptr[L], p1 = lvl_ptr[L + 1];
-#pragma omp parallel for schedule(dynamic, 4) reduction(+ : tot, wild) if (p1 - p0 > 8)
+#pragma omp parallel for schedule(dynamic, 4) reduction(+ : tot, wild) if (par && p1 - p0 > 64)
     for (int p = p0; p < p1; ++p) {
-      Worker &k = workers[(size_t)omp_get_thread_num()];
+      Worker &k = workers[par ? (size_t)omp_get_thread_num() : 0];
       k.w.add(p, 1.0);
       for (int e = irp[p]; e < irp[p + 1]; ++e) {
         const int q = dep[e];

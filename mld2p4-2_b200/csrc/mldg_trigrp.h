@@ -36,7 +36,9 @@ struct TriGroups {
 // no row of either has more than `row`, and every row of W has an absolute sum of at most `growth` (a bound on
 // ||L_gg^{-1}||, so that the explicit inverse is as accurate as the
 // substitution it replaces); a single level is always a group (W = I, V = L).
+// par: rows of a level shared by the OpenMP threads.
 void build_tri_groups(const std::vector<int> &lvl_ptr, const std::vector<int> &irp, const std::vector<int> &dep,
-                      const std::vector<double> &val, int64_t budget, int row, double growth, TriGroups *out);
+                      const std::vector<double> &val, int64_t budget, int row, double growth, bool par,
+                      TriGroups *out);
 
 }  // namespace mldg
