@@ -71,17 +71,20 @@ template <> struct Bits<float> {
 };
 
 // Programmatic dependent launch.  A kernel launched with the programmatic
-// stream-serialization attribute may be scheduled while the kernel before it
-// in the stream is still finishing; pdl_enter() first waits until that
-// kernel has completed and its writes are visible (so it must run before
-// the kernel touches any memory), then allows the next kernel in the stream
-// to be scheduled early in turn.  Both instructions are no-ops in a kernel
-// launched without the attribute.  Every kernel that the host may launch
-// with the attribute calls it first, so completion stays transitive along
-// the stream.
+// stream-serialization attribute may be scheduled once every block of the
+// kernel before it in the stream has called pdl_launch; pdl_wait() waits until
+// that kernel has completed and its writes are visible, so it must run before
+// the kernel touches any memory that a kernel writes.  What never changes after
+// finalize (the matrices: row pointers, offsets, indices, values, scales) may be
+// read before it, so that a kernel's first matrix loads are in flight while the
+// kernel before it finishes.  Every kernel waits before it ends, so completion
+// stays transitive along the stream.  Both instructions are no-ops in a kernel
+// launched without the attribute.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_launch();
+  pdl_wait();
 }
 
 // Spin-wait limits: a wait that exceeds kSpinLimit polls records
@@ -202,6 +205,99 @@ __device__ __forceinline__ T csr_lane_sum(int k0, int e, int row, const CI *__re
   return s;
 }
 
+// Rows of a CSR kernel: TPR lanes a row, each warp walking 32/TPR rows a step.
+// The first step's row pointers and first batch of entries are loaded before
+// pdl_wait; ep(row) loads what the epilogue needs ahead of the gathers;
+// done(row, sum, ep's value) runs in the first lane of each row.
+template <typename T, int TPR, typename CI, typename V, typename G, typename E, typename D>
+__device__ __forceinline__ void csr_rows(int nr, const int *__restrict__ irp, const CI *__restrict__ ja,
+                                         const V *__restrict__ val, G g, E ep, D done) {
+  constexpr int RPW = 32 / TPR, U = CsrU<TPR>::value;
+  const int lane = threadIdx.x & 31, sub = lane % TPR, grp = lane / TPR;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  T vv[U];
+  int jj[U], k = 0, e = 0, row = 0;
+  auto batch = [&]() {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int kk = k + u * TPR;
+      const bool ok = kk < e;
+      vv[u] = ok ? ldval<T>(val, kk) : T(0);
+      jj[u] = ok ? colof(ja, kk, row) : 0;
+    }
+  };
+  auto fetch = [&](int r0) {
+    row = r0 + grp;
+    k = e = 0;
+    if (row < nr) {
+      k = irp[row] + sub;
+      e = irp[row + 1];
+    }
+    batch();
+  };
+  int r0 = warp * RPW;
+  if (r0 < nr) fetch(r0);
+  pdl_wait();
+  while (r0 < nr) {
+    const bool mine = row < nr && sub == 0;
+    const auto op = ep(mine ? row : 0);
+    T s = T(0);
+    for (;;) {
+      T xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = k + u * TPR < e ? g(jj[u]) : T(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k + u * TPR < e) s = fma(vv[u], xv[u], s);
+      k += TPR * U;
+      if (k >= e) break;
+      batch();
+    }
+#pragma unroll
+    for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, TPR);
+    if (mine) done(row, s, op);
+    r0 += nwarps * RPW;
+    if (r0 < nr) fetch(r0);
+  }
+}
+
+// The epilogues' operands, loaded ahead of a row's gathers: b and out of an
+// SpMV; d, x, ty and out of a Jacobi sweep; the row scale of FP16 values.
+template <typename T>
+struct SpmvOps {
+  T b, o;
+  float rs;
+};
+template <typename T, typename V>
+__device__ __forceinline__ SpmvOps<T> spmv_ops(int row, const T *__restrict__ b, const T *out, T a2,
+                                               const float *__restrict__ rs) {
+  return {b ? b[row] : T(0), a2 != T(0) ? out[row] : T(0), std::is_same<V, __half>::value ? __ldg(rs + row) : 0.f};
+}
+template <typename T, typename V>
+__device__ __forceinline__ T spmv_value(T s, const SpmvOps<T> &p, T a1, bool hasb, T a0, T a2) {
+  T r = a1 * row_scaled<T, V>(s, &p.rs, 0);
+  if (hasb) r = fma(a0, p.b, r);
+  if (a2 != T(0)) r = fma(a2, p.o, r);
+  return r;
+}
+template <typename T>
+struct JacOps {
+  T d, x, t, o;
+  float rs;
+};
+template <typename T, typename V>
+__device__ __forceinline__ JacOps<T> jac_ops(int row, const T *__restrict__ d, const T *__restrict__ x,
+                                             const T *__restrict__ ty, int first, T omega, T beta, const T *out,
+                                             const float *__restrict__ rs) {
+  return {d[row], x[row], (!first && omega != T(1)) ? ty[row] : T(0), beta != T(0) ? out[row] : T(0),
+          std::is_same<V, __half>::value ? __ldg(rs + row) : 0.f};
+}
+template <typename T, typename V>
+__device__ __forceinline__ T jac_value(T s, const JacOps<T> &p, int first, T omega, T alpha, T beta) {
+  return jac_row(p.d, p.x, row_scaled<T, V>(s, &p.rs, 0), p.t, first != 0, omega, alpha, beta, p.o);
+}
+
 template <typename T, int TPR, typename CI = int, typename V = T>
 __global__ void __launch_bounds__(256) k_spmv(int nr, const int *__restrict__ irp,
                                               const CI *__restrict__ ja,
@@ -209,27 +305,11 @@ __global__ void __launch_bounds__(256) k_spmv(int nr, const int *__restrict__ ir
                                               const T *__restrict__ v, T a1,
                                               const T *__restrict__ b, T a0, T *out, T a2,
                                               const float *__restrict__ rs = nullptr) {
-  pdl_enter();
-  constexpr int RPW = 32 / TPR;
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % TPR;
-  const int grp = lane / TPR;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int r0 = warp * RPW; r0 < nr; r0 += nwarps * RPW) {
-    const int row = r0 + grp;
-    T s = T(0);
-    if (row < nr)
-      s = csr_lane_sum<T, TPR>(irp[row] + sub, irp[row + 1], row, ja, val, [&](int j) { return __ldg(v + j); });
-#pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, TPR);
-    if (row < nr && sub == 0) {
-      T r = a1 * row_scaled<T, V>(s, rs, row);
-      if (b) r = fma(a0, b[row], r);
-      if (a2 != T(0)) r = fma(a2, out[row], r);
-      out[row] = r;
-    }
-  }
+  pdl_launch();
+  csr_rows<T, TPR>(
+      nr, irp, ja, val, [&](int j) { return __ldg(v + j); },
+      [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
+      [&](int row, T s, const SpmvOps<T> &p) { out[row] = spmv_value<T, V>(s, p, a1, b != nullptr, a0, a2); });
 }
 
 // ---------------------------------------------------------------------------
@@ -289,6 +369,54 @@ __device__ __forceinline__ void sell_rows(const int *__restrict__ soff, const CI
   }
 }
 
+// The rows of a SELL kernel with one slice per warp step: the first slice's
+// first block is loaded before pdl_wait, ep and done as in csr_rows.
+template <typename T, typename CI, typename V, typename F, typename E, typename D>
+__device__ __forceinline__ void sell_loop(int nr, const int *__restrict__ soff, const CI *__restrict__ sj,
+                                          const V *__restrict__ sv, F f, E ep, D done) {
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int ns = (nr + 31) >> 5;
+  T vv[kSellU];
+  int jj[kSellU], e = 0, e1 = 0, row = 0;
+  auto block = [&]() {
+#pragma unroll
+    for (int u = 0; u < kSellU; ++u) {
+      const int k = e + 32 * u;
+      const bool ok = k < e1;
+      vv[u] = ok ? ldval<T>(sv, k) : T(0);
+      jj[u] = ok ? sell_col(sj, k, row) : 0;
+    }
+  };
+  auto fetch = [&](int sl) {
+    row = (sl << 5) + lane;
+    e = __ldg(soff + sl) + lane;
+    e1 = __ldg(soff + sl + 1);
+    block();
+  };
+  int sl = warp;
+  if (sl < ns) fetch(sl);
+  pdl_wait();
+  while (sl < ns) {
+    const auto op = ep(min(row, nr - 1));
+    T acc = T(0);
+    while (e < e1) {
+      T xv[kSellU];
+#pragma unroll
+      for (int u = 0; u < kSellU; ++u) xv[u] = e + 32 * u < e1 ? f(jj[u]) : T(0);
+#pragma unroll
+      for (int u = 0; u < kSellU; ++u)
+        if (e + 32 * u < e1) acc = fma(vv[u], xv[u], acc);
+      e += 32 * kSellU;
+      if (e < e1) block();
+    }
+    if (row < nr) done(row, acc, op);
+    sl += nwarps;
+    if (sl < ns) fetch(sl);
+  }
+}
+
 // out[i] = a0*b[i] + a1*(A v)[i] + a2*out[i]; S slices per warp iteration
 template <typename T, typename CI, int S, typename V = T>
 __global__ void __launch_bounds__(256) k_spmv_sell(int nr, const int *__restrict__ soff,
@@ -296,6 +424,14 @@ __global__ void __launch_bounds__(256) k_spmv_sell(int nr, const int *__restrict
                                                    const T *__restrict__ v, T a1, const T *__restrict__ b,
                                                    T a0, T *out, T a2,
                                                    const float *__restrict__ rs = nullptr) {
+  if constexpr (S == 1) {
+    pdl_launch();
+    sell_loop<T>(
+        nr, soff, sj, sv, [&](int j) { return __ldg(v + j); },
+        [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
+        [&](int row, T s, const SpmvOps<T> &p) { out[row] = spmv_value<T, V>(s, p, a1, b != nullptr, a0, a2); });
+    return;
+  }
   pdl_enter();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -430,6 +566,18 @@ __global__ void __launch_bounds__(256) k_jacobi_sell(int nr, const int *__restri
                                                      const T *__restrict__ d, const T *__restrict__ x,
                                                      const T *__restrict__ ty, int first, T omega, T alpha,
                                                      T beta, T *out, const float *__restrict__ rs = nullptr) {
+  if constexpr (S == 1) {
+    pdl_launch();
+    auto ep = [&](int row) { return jac_ops<T, V>(row, d, x, ty, first, omega, beta, out, rs); };
+    auto done = [&](int row, T s, const JacOps<T> &p) { out[row] = jac_value<T, V>(s, p, first, omega, alpha, beta); };
+    if (first == 2)
+      sell_loop<T>(nr, soff, sj, sv, [&](int j) { return omega * __ldg(x + j); }, ep, done);
+    else if (first)
+      sell_loop<T>(nr, soff, sj, sv, [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, ep, done);
+    else
+      sell_loop<T>(nr, soff, sj, sv, [&](int j) { return __ldg(ty + j); }, ep, done);
+    return;
+  }
   pdl_enter();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -476,8 +624,8 @@ __global__ void __launch_bounds__(256) k_jacobi_sell(int nr, const int *__restri
 // rows of a coarse level (more loads in flight per pass); the autotuner
 // times both.
 template <typename T, int U>
-struct HdiaMinBlocks {  // 256-thread blocks per SM: 32 registers (FP32), 40 (FP64); U = 16 unbounded
-  static constexpr int value = U > 4 ? 1 : (sizeof(T) == 8 ? 6 : 8);
+struct HdiaMinBlocks {  // 256-thread blocks per SM: 40 registers (FP32), 48 (FP64); U = 16 unbounded
+  static constexpr int value = U > 4 ? 1 : (sizeof(T) == 8 ? 5 : 6);
 };
 
 template <typename T, int U = 4, typename F, typename V>
@@ -503,27 +651,64 @@ __device__ __forceinline__ T hdia_row(const int *__restrict__ dptr, const int *_
   return acc;
 }
 
+// The rows of an HDIA kernel (a warp per slice): the first slice's first pass
+// is loaded before pdl_wait, ep and done as in csr_rows.
+template <typename T, int U, typename V, typename F, typename E, typename D>
+__device__ __forceinline__ void hdia_rows(int nr, const int *__restrict__ dptr, const int *__restrict__ doff,
+                                          const V *__restrict__ hv, F f, E ep, D done) {
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int ns = (nr + 31) >> 5;
+  T vv[U];
+  int off[U], k = 0, k1 = 0;
+  auto pass = [&]() {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const bool ok = k + u < k1;
+      off[u] = ok ? __ldg(doff + k + u) : 0;
+      vv[u] = ok ? ldval<T>(hv, ((k + u) << 5) + lane) : T(0);
+    }
+  };
+  auto fetch = [&](int sl) {
+    k = __ldg(dptr + sl);
+    k1 = __ldg(dptr + sl + 1);
+    pass();
+  };
+  int sl = warp;
+  if (sl < ns) fetch(sl);
+  pdl_wait();
+  while (sl < ns) {
+    const int row = (sl << 5) + lane;
+    const auto op = ep(min(row, nr - 1));
+    T acc = T(0);
+    while (k < k1) {
+      T xv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) xv[u] = k + u < k1 ? f(min(max(row + off[u], 0), nr - 1)) : T(0);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (k + u < k1) acc = fma(vv[u], xv[u], acc);
+      k += U;
+      if (k < k1) pass();
+    }
+    if (row < nr) done(row, acc, op);
+    sl += nwarps;
+    if (sl < ns) fetch(sl);
+  }
+}
+
 // out[i] = a0*b[i] + a1*(A v)[i] + a2*out[i] on the HDIA copy of A
 template <typename T, typename V = T, int U = 4>
 __global__ void __launch_bounds__(256, (HdiaMinBlocks<T, U>::value))
     k_spmv_hdia(int nr, const int *__restrict__ dptr, const int *__restrict__ doff, const V *__restrict__ hv,
                 const T *__restrict__ v, T a1, const T *__restrict__ b, T a0, T *out, T a2,
                 const float *__restrict__ rs = nullptr) {
-  pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int ns = (nr + 31) >> 5;
-  for (int sl = warp; sl < ns; sl += nwarps) {
-    const int row = (sl << 5) + lane;
-    const T acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane, [&](int j) { return __ldg(v + j); });
-    if (row < nr) {
-      T r = a1 * row_scaled<T, V>(acc, rs, row);
-      if (b) r = fma(a0, b[row], r);
-      if (a2 != T(0)) r = fma(a2, out[row], r);
-      out[row] = r;
-    }
-  }
+  pdl_launch();
+  hdia_rows<T, U>(
+      nr, dptr, doff, hv, [&](int j) { return __ldg(v + j); },
+      [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
+      [&](int row, T s, const SpmvOps<T> &p) { out[row] = spmv_value<T, V>(s, p, a1, b != nullptr, a0, a2); });
 }
 
 // the point-Jacobi sweep of k_jacobi on the HDIA copy of ND
@@ -532,26 +717,15 @@ __global__ void __launch_bounds__(256, (HdiaMinBlocks<T, U>::value))
     k_jacobi_hdia(int nr, const int *__restrict__ dptr, const int *__restrict__ doff, const V *__restrict__ hv,
                   const T *__restrict__ d, const T *__restrict__ x, const T *__restrict__ ty, int first, T omega,
                   T alpha, T beta, T *out, const float *__restrict__ rs = nullptr) {
-  pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int ns = (nr + 31) >> 5;
-  for (int sl = warp; sl < ns; sl += nwarps) {
-    const int row = (sl << 5) + lane;
-    T acc;
-    if (first == 2)
-      acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane, [&](int j) { return omega * __ldg(x + j); });
-    else if (first)
-      acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane,
-                           [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); });
-    else
-      acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane, [&](int j) { return __ldg(ty + j); });
-    if (row < nr)
-      out[row] = jac_row(d[row], x[row], row_scaled<T, V>(acc, rs, row),
-                         (!first && omega != T(1)) ? ty[row] : T(0), first != 0, omega, alpha, beta,
-                         beta != T(0) ? out[row] : T(0));
-  }
+  pdl_launch();
+  auto ep = [&](int row) { return jac_ops<T, V>(row, d, x, ty, first, omega, beta, out, rs); };
+  auto done = [&](int row, T s, const JacOps<T> &p) { out[row] = jac_value<T, V>(s, p, first, omega, alpha, beta); };
+  if (first == 2)
+    hdia_rows<T, U>(nr, dptr, doff, hv, [&](int j) { return omega * __ldg(x + j); }, ep, done);
+  else if (first)
+    hdia_rows<T, U>(nr, dptr, doff, hv, [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, ep, done);
+  else
+    hdia_rows<T, U>(nr, dptr, doff, hv, [&](int j) { return __ldg(ty + j); }, ep, done);
 }
 
 // FP16-valued prolongator with an FP32 per-row scale (precision form):
@@ -603,31 +777,15 @@ __global__ void __launch_bounds__(256) k_jacobi(int nr, const int *__restrict__ 
                                                 const T *__restrict__ ty, int first,
                                                 T omega, T alpha, T beta, T *out,
                                                 const float *__restrict__ rs = nullptr) {
-  pdl_enter();
-  constexpr int RPW = 32 / TPR;
-  const int lane = threadIdx.x & 31;
-  const int sub = lane % TPR;
-  const int grp = lane / TPR;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (int r0 = warp * RPW; r0 < nr; r0 += nwarps * RPW) {
-    const int row = r0 + grp;
-    T s = T(0);
-    if (row < nr) {
-      const int k0 = irp[row] + sub, e = irp[row + 1];
-      if (first == 2)
-        s = csr_lane_sum<T, TPR>(k0, e, row, ja, val, [&](int j) { return omega * __ldg(x + j); });
-      else if (first)
-        s = csr_lane_sum<T, TPR>(k0, e, row, ja, val, [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); });
-      else
-        s = csr_lane_sum<T, TPR>(k0, e, row, ja, val, [&](int j) { return __ldg(ty + j); });
-    }
-#pragma unroll
-    for (int o = TPR / 2; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, TPR);
-    if (row < nr && sub == 0)
-      out[row] = jac_row(d[row], x[row], row_scaled<T, V>(s, rs, row), (!first && omega != T(1)) ? ty[row] : T(0),
-                         first != 0, omega, alpha, beta, beta != T(0) ? out[row] : T(0));
-  }
+  pdl_launch();
+  auto ep = [&](int row) { return jac_ops<T, V>(row, d, x, ty, first, omega, beta, out, rs); };
+  auto done = [&](int row, T s, const JacOps<T> &p) { out[row] = jac_value<T, V>(s, p, first, omega, alpha, beta); };
+  if (first == 2)
+    csr_rows<T, TPR>(nr, irp, ja, val, [&](int j) { return omega * __ldg(x + j); }, ep, done);
+  else if (first)
+    csr_rows<T, TPR>(nr, irp, ja, val, [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, ep, done);
+  else
+    csr_rows<T, TPR>(nr, irp, ja, val, [&](int j) { return __ldg(ty + j); }, ep, done);
 }
 
 // Dense coarsest-level solve: out = alpha * M x + beta * out with M the
@@ -636,14 +794,27 @@ __global__ void __launch_bounds__(256) k_jacobi(int nr, const int *__restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) k_gemv(int n, const T *__restrict__ M, const T *__restrict__ x,
                                               T alpha, T beta, T *out) {
-  pdl_enter();
+  pdl_launch();
+  constexpr int U = 8;  // entries of the row in flight per lane, the first ones before pdl_wait
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  T m[U];
+  auto load = [&](const T *row, int j) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) m[u] = j + 32 * u < n ? __ldg(row + j + 32 * u) : T(0);
+  };
+  if (warp < n) load(M + (size_t)warp * n, lane);
+  pdl_wait();
   for (int i = warp; i < n; i += nwarps) {
     const T *row = M + (size_t)i * n;
     T s = T(0);
-    for (int j = lane; j < n; j += 32) s = fma(row[j], __ldg(x + j), s);
+    for (int j = lane; j < n; j += 32 * U) {
+      if (j != lane || i != warp) load(row, j);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (j + 32 * u < n) s = fma(m[u], __ldg(x + j + 32 * u), s);
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (lane == 0) {
