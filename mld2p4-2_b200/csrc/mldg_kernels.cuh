@@ -620,12 +620,17 @@ __global__ void __launch_bounds__(256) k_jacobi_sell(int nr, const int *__restri
 // with 8/16-byte accesses, 2 slices per warp, and offsets staged in shared
 // memory per block all ran slower than this one-row-per-thread form, which
 // the register limit of __launch_bounds__ keeps at full occupancy.)
+// (Loading the first pass ahead of pdl_wait, as the CSR and SELL kernels do,
+// holds offsets and values across the wait: with the registers that takes, or
+// with spills, the level-0 kernels ran slower, FCG at idim=80 7.5 ms against
+// 7.2, the application at idim=104 240 us against 225; so did a slice of
+// look-ahead.)
 // U = 4 for slices of a few diagonals (a stencil level), 16 for the long
 // rows of a coarse level (more loads in flight per pass); the autotuner
 // times both.
 template <typename T, int U>
-struct HdiaMinBlocks {  // 256-thread blocks per SM: 40 registers (FP32), 48 (FP64); U = 16 unbounded
-  static constexpr int value = U > 4 ? 1 : (sizeof(T) == 8 ? 5 : 6);
+struct HdiaMinBlocks {  // 256-thread blocks per SM: 32 registers (FP32), 40 (FP64); U = 16 unbounded
+  static constexpr int value = U > 4 ? 1 : (sizeof(T) == 8 ? 6 : 8);
 };
 
 template <typename T, int U = 4, typename F, typename V>
@@ -651,64 +656,27 @@ __device__ __forceinline__ T hdia_row(const int *__restrict__ dptr, const int *_
   return acc;
 }
 
-// The rows of an HDIA kernel (a warp per slice): the first slice's first pass
-// is loaded before pdl_wait, ep and done as in csr_rows.
-template <typename T, int U, typename V, typename F, typename E, typename D>
-__device__ __forceinline__ void hdia_rows(int nr, const int *__restrict__ dptr, const int *__restrict__ doff,
-                                          const V *__restrict__ hv, F f, E ep, D done) {
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int ns = (nr + 31) >> 5;
-  T vv[U];
-  int off[U], k = 0, k1 = 0;
-  auto pass = [&]() {
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const bool ok = k + u < k1;
-      off[u] = ok ? __ldg(doff + k + u) : 0;
-      vv[u] = ok ? ldval<T>(hv, ((k + u) << 5) + lane) : T(0);
-    }
-  };
-  auto fetch = [&](int sl) {
-    k = __ldg(dptr + sl);
-    k1 = __ldg(dptr + sl + 1);
-    pass();
-  };
-  int sl = warp;
-  if (sl < ns) fetch(sl);
-  pdl_wait();
-  while (sl < ns) {
-    const int row = (sl << 5) + lane;
-    const auto op = ep(min(row, nr - 1));
-    T acc = T(0);
-    while (k < k1) {
-      T xv[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) xv[u] = k + u < k1 ? f(min(max(row + off[u], 0), nr - 1)) : T(0);
-#pragma unroll
-      for (int u = 0; u < U; ++u)
-        if (k + u < k1) acc = fma(vv[u], xv[u], acc);
-      k += U;
-      if (k < k1) pass();
-    }
-    if (row < nr) done(row, acc, op);
-    sl += nwarps;
-    if (sl < ns) fetch(sl);
-  }
-}
-
 // out[i] = a0*b[i] + a1*(A v)[i] + a2*out[i] on the HDIA copy of A
 template <typename T, typename V = T, int U = 4>
 __global__ void __launch_bounds__(256, (HdiaMinBlocks<T, U>::value))
     k_spmv_hdia(int nr, const int *__restrict__ dptr, const int *__restrict__ doff, const V *__restrict__ hv,
                 const T *__restrict__ v, T a1, const T *__restrict__ b, T a0, T *out, T a2,
                 const float *__restrict__ rs = nullptr) {
-  pdl_launch();
-  hdia_rows<T, U>(
-      nr, dptr, doff, hv, [&](int j) { return __ldg(v + j); },
-      [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
-      [&](int row, T s, const SpmvOps<T> &p) { out[row] = spmv_value<T, V>(s, p, a1, b != nullptr, a0, a2); });
+  pdl_enter();
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int ns = (nr + 31) >> 5;
+  for (int sl = warp; sl < ns; sl += nwarps) {
+    const int row = (sl << 5) + lane;
+    const T acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane, [&](int j) { return __ldg(v + j); });
+    if (row < nr) {
+      T r = a1 * row_scaled<T, V>(acc, rs, row);
+      if (b) r = fma(a0, b[row], r);
+      if (a2 != T(0)) r = fma(a2, out[row], r);
+      out[row] = r;
+    }
+  }
 }
 
 // the point-Jacobi sweep of k_jacobi on the HDIA copy of ND
@@ -717,15 +685,26 @@ __global__ void __launch_bounds__(256, (HdiaMinBlocks<T, U>::value))
     k_jacobi_hdia(int nr, const int *__restrict__ dptr, const int *__restrict__ doff, const V *__restrict__ hv,
                   const T *__restrict__ d, const T *__restrict__ x, const T *__restrict__ ty, int first, T omega,
                   T alpha, T beta, T *out, const float *__restrict__ rs = nullptr) {
-  pdl_launch();
-  auto ep = [&](int row) { return jac_ops<T, V>(row, d, x, ty, first, omega, beta, out, rs); };
-  auto done = [&](int row, T s, const JacOps<T> &p) { out[row] = jac_value<T, V>(s, p, first, omega, alpha, beta); };
-  if (first == 2)
-    hdia_rows<T, U>(nr, dptr, doff, hv, [&](int j) { return omega * __ldg(x + j); }, ep, done);
-  else if (first)
-    hdia_rows<T, U>(nr, dptr, doff, hv, [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, ep, done);
-  else
-    hdia_rows<T, U>(nr, dptr, doff, hv, [&](int j) { return __ldg(ty + j); }, ep, done);
+  pdl_enter();
+  const int lane = threadIdx.x & 31;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int ns = (nr + 31) >> 5;
+  for (int sl = warp; sl < ns; sl += nwarps) {
+    const int row = (sl << 5) + lane;
+    T acc;
+    if (first == 2)
+      acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane, [&](int j) { return omega * __ldg(x + j); });
+    else if (first)
+      acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane,
+                           [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); });
+    else
+      acc = hdia_row<T, U>(dptr, doff, hv, sl, row, nr, lane, [&](int j) { return __ldg(ty + j); });
+    if (row < nr)
+      out[row] = jac_row(d[row], x[row], row_scaled<T, V>(acc, rs, row),
+                         (!first && omega != T(1)) ? ty[row] : T(0), first != 0, omega, alpha, beta,
+                         beta != T(0) ? out[row] : T(0));
+  }
 }
 
 // FP16-valued prolongator with an FP32 per-row scale (precision form):
