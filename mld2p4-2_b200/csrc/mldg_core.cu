@@ -1199,6 +1199,7 @@ struct EngineT : Engine {
       T *x[4] = {};
       int *ctr = nullptr;  // one ticket counter per buffer
       int ring = 4, seq = 0;
+      bool refused = false;  // no plan for this width: the level's other solve
       bool built(char trans) const { return (trans == 'N' ? L : Ut).n > 0; }
     } g[6];
     // coarsest level: explicit inverse of its ILU(0) factorisation (and its transpose)
@@ -1685,7 +1686,7 @@ struct EngineT : Engine {
   }
   // whether a block of Kw columns takes the grouped solve on a level
   static bool grp_for(const Lev &L, int Kw) {
-    return L.grp && (Kw <= kGrpCols || L.nnz_l + L.nnz_u > 2 * kGrpWide * (int64_t)L.n);
+    return L.grp && !L.g[Kw == 1 ? 0 : ilog2(Kw)].refused && (Kw <= kGrpCols || L.nnz_l + L.nnz_u > 2 * kGrpWide * (int64_t)L.n);
   }
   void gpair(Lev &L, int Kw, char trans, const T *x, T beta, T *y) {
     auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
@@ -2280,7 +2281,13 @@ struct EngineT : Engine {
           p->error = std::current_exception();
         }
       };
-      for (size_t k = 1; k < hp.size(); ++k) th.emplace_back(run, &hp[k]);
+      size_t k = 1;
+      try {
+        th.reserve(hp.size());
+        for (; k < hp.size(); ++k) th.emplace_back(run, &hp[k]);
+      } catch (const std::exception &) {  // no more threads: plan the rest here
+        for (; k < hp.size(); ++k) run(&hp[k]);
+      }
       run(&hp[0]);
       for (auto &t : th) t.join();
     } else {
@@ -2288,8 +2295,15 @@ struct EngineT : Engine {
     }
     for (auto &p : hp)
       if (p.error) std::rethrow_exception(p.error);
-    for (auto &p : hp)
+    // a plan that would take most of the memory left is not made: the level
+    // keeps its other solve, as where the indices do not reach
+    size_t need = 0, avail = 0, total = 0;
+    for (auto &p : hp) {
       if (!p.ok) return false;
+      need += (size_t)p.tk.slots * (sizeof(T) + 4) + 16 * p.tk.desc.size() + 4 * (size_t)L.n;
+    }
+    MLDG_CUDA(cudaMemGetInfo(&avail, &total));
+    if (need + (size_t)G.ring * L.n * Kw * sizeof(T) > avail / 2) return false;
     for (auto &p : hp) upload_grp(ar, p, Kw);
     if (!G.ctr) {
       for (int b = 0; b < G.ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
@@ -2564,6 +2578,14 @@ struct EngineT : Engine {
     impl_bytes = 0;
     return keep;
   }
+  // K-wide exchange buffers, all-sentinel (bufAm stays so after every solve pair)
+  void exchange_m(Lev &L) {
+    const size_t n = (size_t)std::max(L.n, 1) * mcap;
+    L.bufAm = marena.alloc<T>(n);
+    L.bufBm = marena.alloc<T>(n);
+    k_fill<T><<<blocks_for((int64_t)n), 256, 0, st>>>((int)n, Sentinel<T>::value(), L.bufAm);
+    k_fill<T><<<blocks_for((int64_t)n), 256, 0, st>>>((int)n, Sentinel<T>::value(), L.bufBm);
+  }
   bool ensure_multi(int Kw, char trans) override {
     bool grown = false;
     if (Kw > mcap) {
@@ -2603,11 +2625,7 @@ struct EngineT : Engine {
         MLDG_CUDA(cudaMemsetAsync(L.twm, 0, sizeof(T) * n, st));
         if ((L.kind == MLDG_SMOOTHER_BJAC || L.kind == MLDG_SMOOTHER_FBGS) && !L.minv &&
             !grp_for(L, mcap)) {
-          // exchange buffers start as all-sentinel (bufAm stays so after every solve pair)
-          L.bufAm = marena.alloc<T>(n);
-          L.bufBm = marena.alloc<T>(n);
-          k_fill<T><<<blocks_for((int64_t)n), 256, 0, st>>>((int)n, Sentinel<T>::value(), L.bufAm);
-          k_fill<T><<<blocks_for((int64_t)n), 256, 0, st>>>((int)n, Sentinel<T>::value(), L.bufBm);
+          exchange_m(L);
         }
       }
       grown = true;
@@ -2616,8 +2634,10 @@ struct EngineT : Engine {
     for (auto &L : lv) {
       if ((L.kind != MLDG_SMOOTHER_BJAC && L.kind != MLDG_SMOOTHER_FBGS) || L.minv) continue;
       if (grp_for(L, Kw)) {
-        if (!L.g[ki].built(trans) && !build_grp(L, Kw, trans, marena)) fail(MLDG_ERR_SIZE, "grouped plan too large for %d columns", Kw);
-        continue;
+        if (L.g[ki].built(trans) || build_grp(L, Kw, trans, marena)) continue;
+        L.g[ki].refused = true;
+        grown = true;  // graphs that a width captured with the grouped solve are dropped
+        if (!L.bufAm) exchange_m(L);
       }
       for (DTri<T> *t : {&L.L, &L.U, &L.Ut, &L.Lt}) {
         if (!t->present() && L.kind == MLDG_SMOOTHER_FBGS) continue;

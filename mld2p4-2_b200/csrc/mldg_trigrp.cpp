@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <new>
 
 namespace mldg {
 
@@ -99,10 +100,10 @@ void build_tri_groups(const std::vector<int> &lvl_ptr, const std::vector<int> &i
   // where a row grows beyond its bounds
   auto level = [&](int L, int g0) -> int64_t {
     int64_t tot = 0;
-    int wild = 0;
+    int wild = 0, failed = 0;
     const int p0 = lvl_ptr[L], p1 = lvl_ptr[L + 1];
-#pragma omp parallel for schedule(dynamic, 4) reduction(+ : tot, wild) if (par && p1 - p0 > 64)
-    for (int p = p0; p < p1; ++p) {
+#pragma omp parallel for schedule(dynamic, 4) reduction(+ : tot, wild, failed) if (par && p1 - p0 > 64)
+    for (int p = p0; p < p1; ++p) try {
       Worker &k = workers[par ? (size_t)omp_get_thread_num() : 0];
       k.w.add(p, 1.0);
       for (int e = irp[p]; e < irp[p + 1]; ++e) {
@@ -128,7 +129,10 @@ void build_tri_groups(const std::vector<int> &lvl_ptr, const std::vector<int> &i
       for (int i = 0; i < r.nw; ++i) s += std::fabs(r.w[i].val);
       if (r.nw > 1 && (!(s <= growth) || std::max(r.nv, r.nw) > row)) ++wild;
       tot += r.nv + r.nw;
+    } catch (const std::bad_alloc &) {  // no exception may leave the parallel loop
+      ++failed;
     }
+    if (failed) throw std::bad_alloc();
     return wild ? -1 : tot;
   };
   int64_t held = 0;
