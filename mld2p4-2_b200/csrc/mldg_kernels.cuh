@@ -82,9 +82,21 @@ template <> struct Bits<float> {
 // launched without the attribute.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_enter() {
-  pdl_launch();
+// A small grid lets the next kernel in before it waits itself; a grid of more
+// than four blocks per SM (of 148) only after it, as its own later blocks need
+// the SMs (idim=160 level 0 in FP16 operators, repeated: the residual 45 us
+// this way, 53 the other).
+__device__ __forceinline__ bool pdl_early() { return gridDim.x <= 592; }
+__device__ __forceinline__ void pdl_begin() {
+  if (pdl_early()) pdl_launch();
+}
+__device__ __forceinline__ void pdl_ready() {
   pdl_wait();
+  if (!pdl_early()) pdl_launch();
+}
+__device__ __forceinline__ void pdl_enter() {
+  pdl_begin();
+  pdl_ready();
 }
 
 // Spin-wait limits: a wait that exceeds kSpinLimit polls records
@@ -241,7 +253,7 @@ __device__ __forceinline__ void csr_rows(int nr, const int *__restrict__ irp, co
   };
   int r0 = warp * RPW;
   if (r0 < nr) fetch(r0);
-  pdl_wait();
+  pdl_ready();
   while (r0 < nr) {
     const bool mine = row < nr && sub == 0;
     const auto op = ep(mine ? row : 0);
@@ -308,7 +320,7 @@ __global__ void __launch_bounds__(256) k_spmv(int nr, const int *__restrict__ ir
                                               const T *__restrict__ v, T a1,
                                               const T *__restrict__ b, T a0, T *out, T a2,
                                               const float *__restrict__ rs = nullptr) {
-  pdl_launch();
+  pdl_begin();
   csr_rows<T, TPR>(
       nr, irp, ja, val, [&](int j) { return __ldg(v + j); },
       [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
@@ -400,7 +412,7 @@ __device__ __forceinline__ void sell_loop(int nr, const int *__restrict__ soff, 
   };
   int sl = warp;
   if (sl < ns) fetch(sl);
-  pdl_wait();
+  pdl_ready();
   while (sl < ns) {
     const auto op = ep(min(row, nr - 1));
     T acc = T(0);
@@ -428,7 +440,7 @@ __global__ void __launch_bounds__(256) k_spmv_sell(int nr, const int *__restrict
                                                    T a0, T *out, T a2,
                                                    const float *__restrict__ rs = nullptr) {
   if constexpr (S == 1) {
-    pdl_launch();
+    pdl_begin();
     sell_loop<T>(
         nr, soff, sj, sv, [&](int j) { return __ldg(v + j); },
         [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
@@ -570,7 +582,7 @@ __global__ void __launch_bounds__(256) k_jacobi_sell(int nr, const int *__restri
                                                      const T *__restrict__ ty, int first, T omega, T alpha,
                                                      T beta, T *out, const float *__restrict__ rs = nullptr) {
   if constexpr (S == 1) {
-    pdl_launch();
+    pdl_begin();
     auto ep = [&](int row) { return jac_ops<T, V>(row, d, x, ty, first, omega, beta, out, rs); };
     auto done = [&](int row, T s, const JacOps<T> &p) { out[row] = jac_value<T, V>(s, p, first, omega, alpha, beta); };
     if (first == 2)
@@ -759,7 +771,7 @@ __global__ void __launch_bounds__(256) k_jacobi(int nr, const int *__restrict__ 
                                                 const T *__restrict__ ty, int first,
                                                 T omega, T alpha, T beta, T *out,
                                                 const float *__restrict__ rs = nullptr) {
-  pdl_launch();
+  pdl_begin();
   auto ep = [&](int row) { return jac_ops<T, V>(row, d, x, ty, first, omega, beta, out, rs); };
   auto done = [&](int row, T s, const JacOps<T> &p) { out[row] = jac_value<T, V>(s, p, first, omega, alpha, beta); };
   if (first == 2)
@@ -776,7 +788,7 @@ __global__ void __launch_bounds__(256) k_jacobi(int nr, const int *__restrict__ 
 template <typename T>
 __global__ void __launch_bounds__(256) k_gemv(int n, const T *__restrict__ M, const T *__restrict__ x,
                                               T alpha, T beta, T *out) {
-  pdl_launch();
+  pdl_begin();
   constexpr int U = 8;  // entries of the row in flight per lane, the first ones before pdl_wait
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -787,7 +799,7 @@ __global__ void __launch_bounds__(256) k_gemv(int n, const T *__restrict__ M, co
     for (int u = 0; u < U; ++u) m[u] = j + 32 * u < n ? __ldg(row + j + 32 * u) : T(0);
   };
   if (warp < n) load(M + (size_t)warp * n, lane);
-  pdl_wait();
+  pdl_ready();
   for (int i = warp; i < n; i += nwarps) {
     const T *row = M + (size_t)i * n;
     T s = T(0);
