@@ -472,6 +472,10 @@ constexpr int64_t kGrpBudgetMin = 50000, kGrpBudgetMax = 200000;
 constexpr int kGrpRow = 512;
 constexpr double kGrpGrowth = 64.0;
 constexpr int kGrpCols = 8, kGrpWide = 8;
+// blocks per SM that the grouped solves of a batch of systems share (ms at 1.5,
+// 3, 6, 12: 64 systems of idim 24..96 272, 166, 162, 206, unbounded 620; eight of
+// them 67, 51, 76, 103; the 16 smallest 14.6, 12.3, 15.8, 19.4)
+constexpr double kGrpBatchBlocks = 4.0;
 static int64_t grp_budget(int n, int K) {
   return K > kGrpCols ? kGrpBudgetMin / 2 : K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
 }
@@ -1027,6 +1031,9 @@ struct Engine {
   // while probe or profile events are recorded between kernels, and with
   // MLDG_NO_PDL
   bool pdl = std::getenv("MLDG_NO_PDL") == nullptr;
+  // most blocks of a grouped solve, 0 for no bound: while a batch of systems is
+  // captured, whose solves share the SMs
+  int grp_blocks = 0;
   bool pdl_on() const { return pdl && probe_kind == 0 && !prof; }
   template <typename... KArgs, typename... Args>
   void kl(void (*kern)(KArgs...), int grid, int block, Args... args) {
@@ -1668,7 +1675,9 @@ struct EngineT : Engine {
     a.ctr_reset = G.ctr + 32 * r;
     a.err = err;
     begin(MLDG_KERNEL_TRSV);
-    grp_dispatch(Kw, [&](auto kc) { kl(k_trsv_grp<T, decltype(kc)::value>, g.grid, 256, a); });
+    grp_dispatch(Kw, [&](auto kc) { 
+      kl(k_trsv_grp<T, decltype(kc)::value>, grp_blocks > 0 ? std::min(g.grid, grp_blocks) : g.grid, 256, a);
+    });
     const int64_t vec = (int64_t)g.n * Kw * (int64_t)sizeof(T) * (3 + (out ? 1 + (beta != T(0)) : 0));
     end(g.slots * (int64_t)(sizeof(T) + 4) + 16 * (int64_t)g.m.ntask + vec,
         nnz * (int64_t)(sizeof(T) + 4) + 4 * (2 * (int64_t)g.n + 1) + vec);
@@ -5658,16 +5667,24 @@ static void end_capture_quietly(cudaStream_t st) {
 // scheduled blocks of one system's next kernel would sit on SMs, waiting,
 // that the concurrent branches of the other systems need (64 systems at idim
 // 24..96: 185 ms with it, against 155 ms without).
+// The systems' grouped solves share the SMs by their rows: a solve alone keeps
+// up to three blocks an SM waiting, which 64 systems have no room for.
 struct NoPdlScope {
   std::vector<std::pair<Engine *, bool>> saved;
   NoPdlScope(int nsys, Handle **hs) {
+    double rows = 0;
+    for (int i = 0; i < nsys; ++i) rows += hs[i]->n0;
     for (int i = 0; i < nsys; ++i) {
       saved.emplace_back(hs[i]->eng.get(), hs[i]->eng->pdl);
       hs[i]->eng->pdl = false;
+      hs[i]->eng->grp_blocks = std::max(2, (int)(kGrpBatchBlocks * hs[i]->nsm * hs[i]->n0 / std::max(rows, 1.0)));
     }
   }
   ~NoPdlScope() {
-    for (auto &e : saved) e.first->pdl = e.second;
+    for (auto &e : saved) {
+      e.first->pdl = e.second;
+      e.first->grp_blocks = 0;
+    }
   }
 };
 
