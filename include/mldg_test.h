@@ -63,6 +63,12 @@ int mldg_grp_plan_check(const mldg_csr *T, int upper, const double *scale, const
  * Returns MLDG_SUCCESS or MLDG_ERR_CUDA. */
 int mldg_test_set_spin_limit(int device, int polls);
 
+/* Makes a device allocation of the calling thread fail on the host, after
+ * `after` further ones that do not (negative: none fails).  The failing call
+ * returns MLDG_ERR_ALLOC; a test then repeats it and checks that it is right.
+ * Returns MLDG_SUCCESS. */
+int mldg_test_set_alloc_failure(int after);
+
 #ifdef __cplusplus
 }
 #endif

@@ -150,6 +150,10 @@ struct HostLevel {
   double damp = 1.0;
 };
 
+// Allocations of this thread until one fails on purpose, negative: none does
+// (mldg_test_set_alloc_failure).
+static thread_local int g_alloc_failure = -1;
+
 // ---------------------------------------------------------------------------
 // Device memory arena: everything lives until mldg_destroy.
 struct Arena {
@@ -161,9 +165,12 @@ struct Arena {
     if (n == 0) n = 1;
     // 64 bytes of slack past the end: the staged kernels' bulk copies widen
     // each slice to 16-byte boundaries (mldg_spmv_stg.cuh)
-    cudaError_t e = cudaMalloc(&p, n * sizeof(T) + 64);
-    if (e != cudaSuccess)
+    const bool on_purpose = g_alloc_failure >= 0 && g_alloc_failure-- == 0;
+    const cudaError_t e = on_purpose ? cudaErrorMemoryAllocation : cudaMalloc(&p, n * sizeof(T) + 64);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // the call reports it; the next call on the handle starts clean
       fail(MLDG_ERR_ALLOC, "cudaMalloc(%zu bytes): %s", n * sizeof(T), cudaGetErrorString(e));
+    }
     ptrs.push_back(p);
     bytes += n * sizeof(T);
     return (T *)p;
@@ -996,6 +1003,8 @@ struct Engine {
   // n0 x K interleaved).  ensure_multi allocates the K-wide buffers (true when
   // they were reallocated, which invalidates captured multi graphs).
   virtual bool ensure_multi(int K, char trans) = 0;
+  // gives back all that ensure_multi made: the state before its first call
+  virtual void release_multi() = 0;
   virtual void record_multi(char trans, int K) = 0;
   double *xin_m = nullptr, *yout_m = nullptr, *col_m = nullptr;
   int mcap = 0;
@@ -2595,20 +2604,26 @@ struct EngineT : Engine {
     k_fill<T><<<blocks_for((int64_t)n), 256, 0, st>>>((int)n, Sentinel<T>::value(), L.bufAm);
     k_fill<T><<<blocks_for((int64_t)n), 256, 0, st>>>((int)n, Sentinel<T>::value(), L.bufBm);
   }
+  void release_multi() override {
+    marena.release();
+    mcap = 0;
+    xin_m = yout_m = col_m = nullptr;
+    for (auto &L : lv) {
+      L.xm = L.ym = L.tym = L.twm = L.tzm = L.bufAm = L.bufBm = nullptr;
+      L.gflip_m = 0;
+      for (int q = 1; q < 6; ++q) L.g[q] = typename Lev::Grp();
+      for (DTri<T> *t : {&L.L, &L.U, &L.Ut, &L.Lt})
+        for (int q = 1; q < 6; ++q) {  // [0] (one column) lives in the main arena
+          t->blkm[q] = nullptr;
+          t->nblkm[q] = t->gridm[q] = 0;
+          t->ell[q] = typename DTri<T>::Ell();
+        }
+    }
+  }
   bool ensure_multi(int Kw, char trans) override {
     bool grown = false;
     if (Kw > mcap) {
-      marena.release();
-      for (auto &L : lv) {
-        L.xm = L.ym = L.tym = L.twm = L.tzm = L.bufAm = L.bufBm = nullptr;
-        for (int q = 1; q < 6; ++q) L.g[q] = typename Lev::Grp();
-        for (DTri<T> *t : {&L.L, &L.U, &L.Ut, &L.Lt})
-          for (int q = 1; q < 6; ++q) {  // [0] (one column) lives in the main arena
-            t->blkm[q] = nullptr;
-            t->nblkm[q] = t->gridm[q] = 0;
-            t->ell[q] = typename DTri<T>::Ell();
-          }
-      }
+      release_multi();
       mcap = Kw;
       const size_t n0 = (size_t)std::max(lv[0].n, 1);
       if ((int64_t)n0 * mcap >= (int64_t)INT32_MAX) fail(MLDG_ERR_SIZE, "n * nrhs too large");
@@ -5061,8 +5076,17 @@ static int width_for(int k) {
   while (K < k) K *= 2;
   return K;
 }
+// Buffers and plans for K columns.  Where an allocation fails, the graphs that
+// hold the old ones and whatever was half made go, so that the next call
+// starts over.
 static void prepare_multi(Handle *h, int K, char trans) {
-  if (h->eng->ensure_multi(K, trans)) drop_multi_graphs(h);
+  try {
+    if (h->eng->ensure_multi(K, trans)) drop_multi_graphs(h);
+  } catch (...) {
+    drop_multi_graphs(h);
+    h->eng->release_multi();
+    throw;
+  }
 }
 
 // nrhs > 1: blocks of up to 32 columns through the K-wide V-cycle
@@ -6607,6 +6631,11 @@ extern "C" int mldg_test_set_spin_limit(int device, int polls) {
   if (cudaSetDevice(device) != cudaSuccess) return MLDG_ERR_CUDA;
   if (cudaMemcpyToSymbol(mldg::g_spin_limit, &v, sizeof(int)) != cudaSuccess) return MLDG_ERR_CUDA;
   return cudaDeviceSynchronize() == cudaSuccess ? MLDG_SUCCESS : MLDG_ERR_CUDA;
+}
+
+extern "C" int mldg_test_set_alloc_failure(int after) {
+  mldg::g_alloc_failure = after;
+  return MLDG_SUCCESS;
 }
 
 extern "C" int mldg_blk_plan_check(const mldg_csr *Tc, int upper, const double *scale, const double *rhs,
