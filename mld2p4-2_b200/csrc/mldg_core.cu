@@ -1976,10 +1976,11 @@ struct EngineT : Engine {
   bool kcycle_mode() const { return cycle == MLDG_CYCLE_K || cycle == MLDG_CYCLE_KSYM; }
   void ensure_k() {
     if (!kvec.empty()) return;
-    kvec.resize(lv.size());
+    karena.release();  // of a call whose allocations failed
+    std::vector<KVec> made(lv.size());
     for (size_t l = 0; l < lv.size(); ++l) {
       const size_t n = (size_t)std::max(lv[l].n, 1);
-      KVec &k = kvec[l];
+      KVec &k = made[l];
       k.w = karena.alloc<T>(n);
       k.v = karena.alloc<T>(n);
       k.v1 = karena.alloc<T>(n);
@@ -1989,7 +1990,8 @@ struct EngineT : Engine {
     }
     kpart = karena.alloc<double>(3 * kRedBlocks);
     kres = karena.alloc<double>(4);
-    MLDG_CUDA(cudaMallocHost(&khost, 4 * sizeof(double)));
+    if (!khost) MLDG_CUDA(cudaMallocHost(&khost, 4 * sizeof(double)));
+    kvec = std::move(made);
   }
   void copy(int n, const T *x, T *y) { k_axpby_impl(n, x, T(0), y); }
   void axpby2(int n, T a, const T *x, T b, T *y) {
@@ -5506,6 +5508,7 @@ static void ensure_krylov_m(Handle *h, int K) {
   if (!h->hksc_m) MLDG_CUDA(cudaMallocHost(&h->hksc_m, sizeof(KrylovM)));
   if (K <= h->kcap) return;
   h->karena.release();
+  h->kcap = 0;  // until every vector is there
   const size_t nk = (size_t)std::max(h->n0, 1) * K;
   h->kb_m = h->karena.alloc<double>(nk);
   h->kx_m = h->karena.alloc<double>(nk);

@@ -83,3 +83,50 @@ def test_block(mld, orc, smoother, trans, width):
             state["h"].apply_block(X.copy(), trans=trans)
         _fail_after(mld, -1)
         _close(state["h"].apply_block(X[:2].copy(), trans=trans), ref[:2])
+
+
+def test_krylov_vectors(mld, orc):
+    """The vectors of a block solve: grown for a wider block, the allocation
+    fails, and a narrower solve follows on the same handle; and the vectors of
+    the K-cycle."""
+    a = orc.gen_pde3d(9, 1, ISO)
+    op = orc.Prec(oracle_params(orc, "BJAC", mcs=100))
+    op.build(a)
+    B = np.array([orc.spmv(a, np.full(a.nrows, 1.0 + k)) for k in range(9)])
+    ones = np.array([np.full(a.nrows, 1.0 + k) for k in range(9)])
+    state = {}
+
+    def solve(k):
+        return state["h"].krylov_multi("FCG", B[:k].copy(), eps=1e-12)[0]
+
+    def new():
+        state["h"] = upload_oracle_hierarchy(mld, orc, op, autotune=False)
+        state["h"].apply_block(np.zeros((16, a.nrows)))  # the block's own buffers are there
+        assert np.max(np.abs(solve(2) / ones[:2] - 1)) < 1e-9
+
+    n = 0
+    while True:
+        new()
+        _fail_after(mld, n)
+        try:
+            solve(9)
+            break
+        except mld.MldError as e:
+            assert e.code == ERR_ALLOC
+        finally:
+            _fail_after(mld, -1)
+        assert np.max(np.abs(solve(2) / ones[:2] - 1)) < 1e-9  # the narrower solve first
+        assert np.max(np.abs(solve(9) / ones - 1)) < 1e-9
+        n += 1
+    assert n >= 4
+    x = np.random.default_rng(3).uniform(-1, 1, a.nrows)
+    h = upload_oracle_hierarchy(mld, orc, op, autotune=False)
+    h.set_cycle(2)
+    ref = h.apply(x)
+
+    def kcycle():
+        state["h"] = upload_oracle_hierarchy(mld, orc, op, autotune=False)
+        state["h"].set_cycle(2)
+
+    n = _each_allocation(mld, lambda: [state["h"].apply(x)], lambda y: _close(y, [ref]), kcycle)
+    assert n >= 4
