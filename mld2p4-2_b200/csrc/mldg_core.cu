@@ -4500,7 +4500,8 @@ static Engine *make_engine(Handle *h) {
     clk = now;
   };
   set_trsv_smem_attr<T>();
-  auto *e = new EngineT<T>();
+  auto owner = std::make_unique<EngineT<T>>();
+  EngineT<T> *e = owner.get();
   e->h = h;
   e->st = h->st;
   e->pev0 = h->pev0;
@@ -4847,7 +4848,7 @@ static Engine *make_engine(Handle *h) {
   tick("dense level inverses");
   if (std::getenv("MLDG_TIMING"))
     for (auto &kv : tm) std::fprintf(stderr, "mldg timing: finalize %-32s %.3f s\n", kv.first.c_str(), kv.second);
-  return e;
+  return owner.release();
 }
 
 static void check_level(const HostLevel &H, int l, const HostLevel *prev) {
@@ -4898,6 +4899,7 @@ static void finalize(Handle *h, int nlev, int precision) {
       precision != MLDG_PREC_FP32_H16)
     fail(MLDG_ERR_ARG, "unknown precision %d", precision);
   // drop any previous device state
+  h->finalized = false;
   for (int t = 0; t < 2; ++t)
     if (h->gexec[t]) {
       cudaGraphExecDestroy(h->gexec[t]);

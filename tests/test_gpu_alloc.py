@@ -130,3 +130,26 @@ def test_krylov_vectors(mld, orc):
 
     n = _each_allocation(mld, lambda: [state["h"].apply(x)], lambda y: _close(y, [ref]), kcycle)
     assert n >= 4
+
+
+@pytest.mark.parametrize("smoother", ["BJAC", "FBGS"])
+def test_finalize(mld, orc, smoother):
+    """A hierarchy finalized again whose device data do not fit: the handle is
+    not built (it answers with an error, as before its first finalize), and
+    finalizing it once more mends it."""
+    a = orc.gen_pde3d(9, 1, ISO)
+    op = orc.Prec(oracle_params(orc, smoother, mcs=100))
+    op.build(a)
+    h = upload_oracle_hierarchy(mld, orc, op, autotune=False)
+    x = np.random.default_rng(5).uniform(-1, 1, a.nrows)
+    ref = op.apply(x)
+    for n in (0, 1, 7, 20, 33, 40):
+        _fail_after(mld, n)
+        with pytest.raises(mld.MldError) as e:
+            h.finalize(op.nlev)
+        assert e.value.code == ERR_ALLOC
+        _fail_after(mld, -1)
+        with pytest.raises(mld.MldError):
+            h.apply(x)
+        h.finalize(op.nlev)
+        _close([h.apply(x)], [ref])
