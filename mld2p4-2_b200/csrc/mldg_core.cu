@@ -2554,6 +2554,7 @@ struct EngineT : Engine {
     }
     for (DTri<T> *f : {&L.L, &L.U}) f->ell[ki] = typename DTri<T>::Ell();
     tmp.release();
+    if (!ok) return false;  // no ELL plans to form the inverse with
     // keep the dense form only if it is faster
     auto op = [&]() {
       if (gs) {
