@@ -2322,8 +2322,11 @@ struct EngineT : Engine {
       if (!p.ok) return false;
       need += (size_t)p.tk.slots * (sizeof(T) + 4) + 16 * p.tk.desc.size() + 4 * (size_t)L.n;
     }
+    need += (size_t)G.ring * L.n * Kw * sizeof(T);
     MLDG_CUDA(cudaMemGetInfo(&avail, &total));
-    if (need + (size_t)G.ring * L.n * Kw * sizeof(T) > avail / 2) return false;
+    size_t most = avail / 2;
+    if (const char *e = std::getenv("MLDG_GRP_MB")) most = std::min(most, (size_t)std::max(0, std::atoi(e)) << 20);
+    if (need > most) return false;
     for (auto &p : hp) upload_grp(ar, p, Kw);
     if (!G.ctr) {
       for (int b = 0; b < G.ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
@@ -4571,6 +4574,54 @@ static Engine *make_engine(Handle *h) {
             (H.kind == MLDG_SMOOTHER_FBGS ||
              (H.kind == MLDG_SMOOTHER_BJAC &&
               (L.n <= 65536 || H.L.nnz() <= 8 * (int64_t)L.n || std::getenv("MLDG_NO_REP"))));
+    // level schedules of the four factors: what the other plans are made from,
+    // and the solves that need none (k_trsv_sf, k_trsv_sf_m)
+    if (H.kind == MLDG_SMOOTHER_BJAC) {
+      L.L = build_tri_dev<T>(ar, H.L, false, h->nsm);
+      L.U = build_tri_dev<T>(ar, H.U, true, h->nsm);
+      tick("L, U schedules");
+      HostCSR Lt = transpose(H.L), Ut = transpose(H.U);
+      tick("L^T, U^T transposes");
+      L.Ut = build_tri_dev<T>(ar, Ut, false, h->nsm);  // U^T is lower
+      L.Lt = build_tri_dev<T>(ar, Lt, true, h->nsm);   // L^T is upper
+      if (std::getenv("MLDG_VERBOSE")) {
+        const DTri<T> *ts[4] = {&L.L, &L.U, &L.Ut, &L.Lt};
+        const char *nm[4] = {"L", "U", "Ut", "Lt"};
+        for (int q = 0; q < 4; ++q)
+          std::fprintf(stderr,
+                       "mldg: level %d %-2s n=%d nnz=%lld levels=%d mode=%d tpr=%d e=%d D=%d "
+                       "capR=%d capE=%d smem=%zu grid=%d\n",
+                       l, nm[q], ts[q]->n, (long long)ts[q]->nnz, ts[q]->nlevels, ts[q]->mode,
+                       ts[q]->tpr, ts[q]->e, ts[q]->stg.D, ts[q]->stg.capR, ts[q]->stg.capE,
+                       ts[q]->smem, ts[q]->grid);
+      }
+    }
+    tick("level schedules");
+    std::vector<double> dh = H.d;
+    if (H.kind == MLDG_SMOOTHER_FBGS) {
+      // (D+L)^{-1} and (D+U)^{-1} as unit-triangular solves of the rows
+      // scaled by 1/a_ii, the right-hand side scaled by 1/a_ii
+      for (double &v : dh) v = 1.0 / v;
+      HostCSR Ls = H.L, Us = H.U;
+      for (int i = 0; i < Ls.nr; ++i) {
+        for (int k = Ls.irp[i]; k < Ls.irp[i + 1]; ++k) Ls.val[k] *= dh[i];
+        for (int k = Us.irp[i]; k < Us.irp[i + 1]; ++k) Us.val[k] *= dh[i];
+      }
+      L.L = build_tri_dev<T>(ar, Ls, false, h->nsm);
+      L.U = build_tri_dev<T>(ar, Us, true, h->nsm);
+      if (std::max(H.sweeps_pre, H.sweeps_post) > 1) {
+        // later sweeps: wv = x - U xit (forward) / x - L xit (backward)
+        L.GU = to_dev<T>(ar, H.U);
+        L.GL = to_dev<T>(ar, H.L);
+      }
+    }
+    tick("FBGS factors");
+    // a refused grouped plan leaves the level to its other solves, planned below
+    if (L.grp) {
+      L.h_d = dh;
+      L.grp = e->build_grp(L, 1, 0, ar);
+      tick("grouped plans");
+    }
     if (H.kind == MLDG_SMOOTHER_BJAC && !L.grp && !std::getenv("MLDG_NO_WIN")) {
       const int n = H.A.nr;
       // Single-CTA windows win on small levels; large levels stay on the
@@ -4606,47 +4657,6 @@ static Engine *make_engine(Handle *h) {
       }
     }
     tick("window plans");
-    // level schedules of the four factors: the single-vector solve where no
-    // window plan was taken, and always the multi-RHS solve (k_trsv_sf_m)
-    if (H.kind == MLDG_SMOOTHER_BJAC) {
-      L.L = build_tri_dev<T>(ar, H.L, false, h->nsm);
-      L.U = build_tri_dev<T>(ar, H.U, true, h->nsm);
-      tick("L, U schedules");
-      HostCSR Lt = transpose(H.L), Ut = transpose(H.U);
-      tick("L^T, U^T transposes");
-      L.Ut = build_tri_dev<T>(ar, Ut, false, h->nsm);  // U^T is lower
-      L.Lt = build_tri_dev<T>(ar, Lt, true, h->nsm);   // L^T is upper
-      if (std::getenv("MLDG_VERBOSE") && !L.win) {
-        const DTri<T> *ts[4] = {&L.L, &L.U, &L.Ut, &L.Lt};
-        const char *nm[4] = {"L", "U", "Ut", "Lt"};
-        for (int q = 0; q < 4; ++q)
-          std::fprintf(stderr,
-                       "mldg: level %d %-2s n=%d nnz=%lld levels=%d mode=%d tpr=%d e=%d D=%d "
-                       "capR=%d capE=%d smem=%zu grid=%d\n",
-                       l, nm[q], ts[q]->n, (long long)ts[q]->nnz, ts[q]->nlevels, ts[q]->mode,
-                       ts[q]->tpr, ts[q]->e, ts[q]->stg.D, ts[q]->stg.capR, ts[q]->stg.capE,
-                       ts[q]->smem, ts[q]->grid);
-      }
-    }
-    tick("level schedules");
-    std::vector<double> dh = H.d;
-    if (H.kind == MLDG_SMOOTHER_FBGS) {
-      // (D+L)^{-1} and (D+U)^{-1} as unit-triangular solves of the rows
-      // scaled by 1/a_ii, the right-hand side scaled by 1/a_ii
-      for (double &v : dh) v = 1.0 / v;
-      HostCSR Ls = H.L, Us = H.U;
-      for (int i = 0; i < Ls.nr; ++i) {
-        for (int k = Ls.irp[i]; k < Ls.irp[i + 1]; ++k) Ls.val[k] *= dh[i];
-        for (int k = Us.irp[i]; k < Us.irp[i + 1]; ++k) Us.val[k] *= dh[i];
-      }
-      L.L = build_tri_dev<T>(ar, Ls, false, h->nsm);
-      L.U = build_tri_dev<T>(ar, Us, true, h->nsm);
-      if (std::max(H.sweeps_pre, H.sweeps_post) > 1) {
-        // later sweeps: wv = x - U xit (forward) / x - L xit (backward)
-        L.GU = to_dev<T>(ar, H.U);
-        L.GL = to_dev<T>(ar, H.L);
-      }
-    }
     if (H.ND.present() && L.nnz_nd > 0) {
       if (H.kind == MLDG_SMOOTHER_JACOBI && std::max(H.sweeps_pre, H.sweeps_post) <= 2 &&
           !std::getenv("MLDG_NO_ND_SCALE")) {
@@ -4663,7 +4673,7 @@ static Engine *make_engine(Handle *h) {
         L.NDT = to_dev<T>(ar, transpose(H.ND), h16);
       }
     }
-    tick("FBGS factors, ND");
+    tick("ND");
     if (dense_coarse) {
       std::vector<double> M, MT;
       dense_ilu_inverse(H.L, H.U, H.d, M, MT);
@@ -4758,11 +4768,6 @@ static Engine *make_engine(Handle *h) {
     MLDG_CUDA(cudaMemset(L.y, 0, sizeof(T) * n));
     MLDG_CUDA(cudaMemset(L.ty, 0, sizeof(T) * n));
     MLDG_CUDA(cudaMemset(L.tw, 0, sizeof(T) * n));
-    if (L.grp) {
-      L.h_d = dh;
-      L.grp = e->build_grp(L, 1, 0, ar);
-      tick("grouped plans");
-    }
     if ((H.kind == MLDG_SMOOTHER_BJAC || H.kind == MLDG_SMOOTHER_FBGS) && !L.grp) {
       L.bufA = ar.alloc<T>(n);
       L.bufB = ar.alloc<T>(n);
