@@ -15,7 +15,6 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
-#include <exception>
 #include <map>
 #include <set>
 #include <cstdarg>
@@ -26,7 +25,6 @@
 #include <mutex>
 #include <string>
 #include <type_traits>
-#include <thread>
 #include <vector>
 
 #include <omp.h>
@@ -185,10 +183,14 @@ struct Arena {
   T *upload(const std::vector<T> &v) {
     return upload(v.data(), v.size());
   }
-  void release() {
-    for (void *p : ptrs) cudaFree(p);
-    ptrs.clear();
-    bytes = 0;
+  void release() { release_to({0, 0}); }
+  // what is allocated after mark() is given back by release_to
+  typedef std::pair<size_t, size_t> Mark;
+  Mark mark() const { return {ptrs.size(), bytes}; }
+  void release_to(Mark m) {
+    for (size_t k = m.first; k < ptrs.size(); ++k) cudaFree(ptrs[k]);
+    ptrs.resize(m.first);
+    bytes = m.second;
   }
 };
 
@@ -493,7 +495,7 @@ constexpr int grp_cols(int K) {
 }
 
 // original row of every position, and the dependencies as positions
-static void grp_positions(int n, bool rev, const std::vector<int> &prow, const std::vector<int> &pja, bool par,
+static void grp_positions(int n, bool rev, const std::vector<int> &prow, const std::vector<int> &pja,
                           std::vector<int> &orig, std::vector<int> &dep) {
   std::vector<int> pos((size_t)n);
   orig.resize((size_t)n);
@@ -502,7 +504,7 @@ static void grp_positions(int n, bool rev, const std::vector<int> &prow, const s
     pos[prow[p]] = p;
     orig[p] = rev ? n - 1 - prow[p] : prow[p];
   }
-#pragma omp parallel for schedule(static, 4096) if (par)
+#pragma omp parallel for schedule(static, 4096)
   for (int64_t k = 0; k < (int64_t)dep.size(); ++k) dep[k] = pos[pja[k]];
 }
 
@@ -517,7 +519,7 @@ struct GrpTasks {
 // wcol(c), wscale(c): index in b and factor of W's column position c; false
 // when the slots outgrow the descriptors
 template <typename T, typename FC, typename FS>
-static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, bool par, GrpTasks<T> &out) {
+static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, GrpTasks<T> &out) {
   const int R = 32 / KC, ng = (int)g.gptr.size() - 1;
   auto len = [&](int p) { return (int64_t)std::max(g.row[p].nv, g.row[p].nw); };
   int64_t at = 0;  // slot groups (one int4 of indices each)
@@ -552,7 +554,7 @@ static bool grp_tasks(const TriGroups &g, int KC, FC wcol, FS wscale, bool par, 
     }
   out.idx.reset(new int4[(size_t)std::max<int64_t>(at, 1)]);
   out.val.reset(new T[(size_t)std::max<int64_t>(4 * at, 1)]);
-#pragma omp parallel for schedule(static, 64) if (par)
+#pragma omp parallel for schedule(static, 64)
   for (int64_t k = 0; k < (int64_t)out.desc.size(); ++k) {
     const int4 d = out.desc[k];
     const int lt = d.w & 255, rows = d.w >> 8, tpr = 1 << lt;
@@ -2209,37 +2211,37 @@ struct EngineT : Engine {
 
   // The host side of a factor's grouped plan for Kw columns; W reads the
   // solution of `src` (null: a vector in original order) scaled by `scale` (by
-  // original row, or null).  par: with OpenMP inside.
+  // original row, or null).
   struct GrpHost {
     const DTri<T> *t = nullptr, *src = nullptr;
     const std::vector<double> *scale = nullptr;
     DGrp<T> *dst = nullptr;
     bool ok = false;
-    std::exception_ptr error;
     std::vector<int> orig;
     TriGroups pl;
     GrpTasks<T> tk;
-    void build(int Kw, bool par) {
+    void build(int Kw) {
       const int n = t->n;
       std::vector<int> dep, at;
-      grp_positions(n, t->rev != 0, t->h_prow, t->h_pja, par, orig, dep);
+      grp_positions(n, t->rev != 0, t->h_prow, t->h_pja, orig, dep);
       if (src) {
         at.resize((size_t)n);
         for (int p = 0; p < n; ++p) at[src->rev ? n - 1 - src->h_prow[p] : src->h_prow[p]] = p;
       }
       int64_t budget = grp_budget(n, Kw);
       if (const char *e = std::getenv("MLDG_GRP_B")) budget = std::max(1, std::atoi(e));
-      build_tri_groups(t->h_lvl, t->h_pirp, dep, t->h_pval, budget, kGrpRow, kGrpGrowth, par, &pl);
+      build_tri_groups(t->h_lvl, t->h_pirp, dep, t->h_pval, budget, kGrpRow, kGrpGrowth, &pl);
       ok = grp_tasks<T>(
           pl, grp_cols<T>(Kw), [&](int c) { return src ? at[orig[c]] : orig[c]; },
-          [&](int c) { return scale ? (*scale)[orig[c]] : 1.0; }, par, tk);
+          [&](int c) { return scale ? (*scale)[orig[c]] : 1.0; }, tk);
     }
+    size_t bytes() const { return (size_t)tk.slots * (sizeof(T) + 4) + 16 * tk.desc.size() + 4 * orig.size(); }
   };
-  // its device side; the host's copies are released
-  void upload_grp(Arena &ar, GrpHost &hp, int Kw) {
+  // its device side
+  DGrp<T> upload_grp(Arena &ar, const GrpHost &hp, int Kw) {
     const DTri<T> &t = *hp.t;
-    DGrp<T> &g = *hp.dst;
-    GrpTasks<T> &tk = hp.tk;
+    DGrp<T> g;
+    const GrpTasks<T> &tk = hp.tk;
     const int n = t.n, KC = grp_cols<T>(Kw);
     g.n = n;
     g.slots = tk.slots;
@@ -2262,14 +2264,30 @@ struct EngineT : Engine {
     if (std::getenv("MLDG_VERBOSE"))
       std::fprintf(stderr, "mldg: grp K=%d n=%d levels=%d groups=%d entries %lld slots %lld tasks %d grid %d occ %d\n", Kw, n,
                    t.nlevels, ng, (long long)hp.pl.entries, (long long)g.slots, g.m.ntask, g.grid, nb);
-    hp = GrpHost();
+    return g;
   }
   // The grouped plans (of trans 'N' or 'T', or of both: 0) and work vectors of a
-  // level for Kw columns.  A small
-  // level's factors are planned by a thread each (their levels are too narrow to
-  // share), a large one's in turn by all threads.
+  // level for Kw columns; false where they are refused.  All or nothing: what
+  // a refusal or a failed allocation leaves behind is given back, and the level
+  // sees the plans only when all are there.
   bool build_grp(Lev &L, int Kw, char trans, Arena &ar) {
     auto &G = L.g[Kw == 1 ? 0 : ilog2(Kw)];
+    const typename Lev::Grp before = G;
+    const Arena::Mark mark = ar.mark();
+    auto undo = [&]() {
+      ar.release_to(mark);
+      G = before;
+    };
+    try {
+      if (try_grp(L, G, Kw, trans, ar)) return true;
+    } catch (...) {
+      undo();
+      throw;
+    }
+    undo();
+    return false;
+  }
+  bool try_grp(Lev &L, typename Lev::Grp &G, int Kw, char trans, Arena &ar) {
     std::vector<GrpHost> hp;
     auto add = [&](const DTri<T> &t, const DTri<T> *src, const std::vector<double> *scale, DGrp<T> &dst) {
       hp.emplace_back();
@@ -2278,8 +2296,9 @@ struct EngineT : Engine {
       hp.back().scale = scale;
       hp.back().dst = &dst;
     };
-    if (L.kind == MLDG_SMOOTHER_FBGS) {
-      G.ring = 2;
+    const bool gs = L.kind == MLDG_SMOOTHER_FBGS;
+    const int ring = gs ? 2 : 4;
+    if (gs) {
       add(L.L, nullptr, &L.h_d, G.L);
       add(L.U, nullptr, &L.h_d, G.U);
     } else {
@@ -2292,44 +2311,24 @@ struct EngineT : Engine {
         add(L.Lt, &L.Ut, &L.h_d, G.Lt);
       }
     }
-    if (L.n <= 262144) {
-      std::vector<std::thread> th;
-      auto run = [Kw](GrpHost *p) {
-        try {
-          p->build(Kw, false);
-        } catch (...) {
-          p->error = std::current_exception();
-        }
-      };
-      size_t k = 1;
-      try {
-        th.reserve(hp.size());
-        for (; k < hp.size(); ++k) th.emplace_back(run, &hp[k]);
-      } catch (const std::exception &) {  // no more threads: plan the rest here
-        for (; k < hp.size(); ++k) run(&hp[k]);
-      }
-      run(&hp[0]);
-      for (auto &t : th) t.join();
-    } else {
-      for (auto &p : hp) p.build(Kw, true);
-    }
-    for (auto &p : hp)
-      if (p.error) std::rethrow_exception(p.error);
     // a plan that would take most of the memory left is not made: the level
-    // keeps its other solve, as where the indices do not reach
-    size_t need = 0, avail = 0, total = 0;
-    for (auto &p : hp) {
-      if (!p.ok) return false;
-      need += (size_t)p.tk.slots * (sizeof(T) + 4) + 16 * p.tk.desc.size() + 4 * (size_t)L.n;
-    }
-    need += (size_t)G.ring * L.n * Kw * sizeof(T);
+    // keeps its other solve, as where the indices do not reach.  One factor after
+    // the other, each on the host only until it is uploaded.
+    size_t need = (size_t)ring * L.n * Kw * sizeof(T), avail = 0, total = 0;
     MLDG_CUDA(cudaMemGetInfo(&avail, &total));
     size_t most = avail / 2;
     if (const char *e = std::getenv("MLDG_GRP_MB")) most = std::min(most, (size_t)std::max(0, std::atoi(e)) << 20);
-    if (need > most) return false;
-    for (auto &p : hp) upload_grp(ar, p, Kw);
+    for (auto &p : hp) {
+      p.build(Kw);
+      need += p.bytes();
+      if (!p.ok || need > most) return false;
+      *p.dst = upload_grp(ar, p, Kw);
+      p.pl = TriGroups();
+      p.tk = GrpTasks<T>();
+    }
     if (!G.ctr) {
-      for (int b = 0; b < G.ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
+      G.ring = ring;
+      for (int b = 0; b < ring; ++b) G.x[b] = ar.alloc<T>((size_t)L.n * Kw);
       G.ctr = ar.alloc<int>(32 * 4);
       reset_grp(L, Kw);
     }
@@ -6686,10 +6685,10 @@ extern "C" int mldg_grp_plan_check(const mldg_csr *Tc, int upper, const double *
     mldg::TriSchedule s;
     mldg::build_tri_schedule(m.nr, m.irp.data(), m.ja.data(), m.val.data(), upper != 0, m.nr, &s);
     std::vector<int> orig, dep;
-    mldg::grp_positions(m.nr, upper != 0, s.prow, s.pja, true, orig, dep);
+    mldg::grp_positions(m.nr, upper != 0, s.prow, s.pja, orig, dep);
     mldg::TriGroups g;
     mldg::build_tri_groups(s.lvl_ptr, s.pirp, dep, s.pval, budget > 0 ? budget : mldg::grp_budget(m.nr, ncols),
-                           row > 0 ? row : mldg::kGrpRow, growth > 0 ? growth : mldg::kGrpGrowth, true, &g);
+                           row > 0 ? row : mldg::kGrpRow, growth > 0 ? growth : mldg::kGrpGrowth, &g);
     const std::vector<double> r(rhs, rhs + m.nr);
     std::vector<double> x;
     auto run = [&](auto tag) {
@@ -6697,7 +6696,7 @@ extern "C" int mldg_grp_plan_check(const mldg_csr *Tc, int upper, const double *
       const int KC = mldg::grp_cols<TT>(ncols);
       mldg::GrpTasks<TT> tk;
       const bool ok = mldg::grp_tasks<TT>(
-          g, KC, [&](int c) { return orig[c]; }, [&](int c) { return scale ? scale[orig[c]] : 1.0; }, true, tk);
+          g, KC, [&](int c) { return orig[c]; }, [&](int c) { return scale ? scale[orig[c]] : 1.0; }, tk);
       stats[0] = ok ? mldg::grp_emulate<TT>(g, tk, KC, r, x) : -1;
       stats[1] = (long long)s.lvl_ptr.size() - 1;
       stats[2] = (long long)g.gptr.size() - 1;
