@@ -481,10 +481,17 @@ constexpr int64_t kGrpBudgetMin = 50000, kGrpBudgetMax = 200000;
 constexpr int kGrpRow = 512;
 constexpr double kGrpGrowth = 64.0;
 constexpr int kGrpCols = 8, kGrpWide = 8;
-// blocks per SM that the grouped solves of a batch of systems share (ms at 1.5,
-// 3, 6, 12: 64 systems of idim 24..96 272, 166, 162, 206, unbounded 620; eight of
-// them 67, 51, 76, 103; the 16 smallest 14.6, 12.3, 15.8, 19.4)
+// Blocks per SM that the grouped solves of a batch of systems share by their
+// rows, and the fewest of a system: a small one of many, left with two, was
+// slower than its level-by-level solve.  ms at 2.5, 3, 4, 5, 6 blocks per SM, at
+// least two: 64 systems of idim 24..96 201, 180, 174, 165, 154 (unbounded 620);
+// eight of them 55, 53, 52, 59, 68; 24 of them 95, 88, 81, 87, 92.  At four per SM
+// and at least 2, 4, 6, 8, 10: the 64 systems 174, 136, 139, 141, 143 (by level,
+// before the grouped solves, 149-156); 64 of idim 24..44 38.0, 35.4, 32.4, 32.3,
+// 33.2 (by level 31.7); 128 of them 69, 56, 55, 56, 56 (by level 48); 64 of idim
+// 40..72 96, 89, 83, 85, 87 (by level 88).
 constexpr double kGrpBatchBlocks = 4.0;
+constexpr int kGrpBatchLeast = 6;
 static int64_t grp_budget(int n, int K) {
   return K > kGrpCols ? kGrpBudgetMin / 2 : K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
 }
@@ -5711,7 +5718,7 @@ struct NoPdlScope {
     for (int i = 0; i < nsys; ++i) {
       saved.emplace_back(hs[i]->eng.get(), hs[i]->eng->pdl);
       hs[i]->eng->pdl = false;
-      hs[i]->eng->grp_blocks = std::max(2, (int)(kGrpBatchBlocks * hs[i]->nsm * hs[i]->n0 / std::max(rows, 1.0)));
+      hs[i]->eng->grp_blocks = std::max(kGrpBatchLeast, (int)(kGrpBatchBlocks * hs[i]->nsm * hs[i]->n0 / std::max(rows, 1.0)));
     }
   }
   ~NoPdlScope() {
