@@ -492,6 +492,9 @@ constexpr int kGrpCols = 8, kGrpWide = 8;
 // 40..72 96, 89, 83, 85, 87 (by level 88).
 constexpr double kGrpBatchBlocks = 4.0;
 constexpr int kGrpBatchLeast = 6;
+// blocks per SM that solves share which run at once without a batch, as the
+// kernel finds them (g_grp_running)
+constexpr int kGrpShareBlocks = 2;
 static int64_t grp_budget(int n, int K) {
   return K > kGrpCols ? kGrpBudgetMin / 2 : K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
 }
@@ -1692,6 +1695,8 @@ struct EngineT : Engine {
     a.ctr = G.ctr + 32 * s;
     a.ctr_reset = G.ctr + 32 * r;
     a.err = err;
+    a.share = grp_blocks > 0 ? 0 : kGrpShareBlocks * nsm;
+    a.least = kGrpBatchLeast;
     begin(MLDG_KERNEL_TRSV);
     grp_dispatch(Kw, [&](auto kc) { 
       kl(k_trsv_grp<T, decltype(kc)::value>, grp_blocks > 0 ? std::min(g.grid, grp_blocks) : g.grid, 256, a);

@@ -23,13 +23,16 @@
 // wait, then V's by ascending position, so that the newest dependencies come
 // last.
 //
-// Warps claim tasks in group order from a ticket counter (one ahead), so the
+// Warps claim tasks in group order from a ticket counter (two ahead: the next
+// task's descriptor is loaded, the one after it claimed), so the
 // lowest unfinished task always runs and every wait ends, whichever blocks are
 // resident; rows of a task belong to one group and never wait on one another.
 // A value of x is its own flag: it holds the sentinel until it is written.
 // Each solve puts the sentinel (and a zero ticket counter) back into buffers
 // that an earlier solve is finished with, so no separate pass does.
 #pragma once
+
+#include <climits>
 
 #include "mldg_multi.cuh"
 
@@ -55,7 +58,20 @@ struct GrpArgs {
   T alpha, beta;
   int *ctr, *ctr_reset;
   int *err;
+  int share, least;  // blocks that the solves running at once share (0: keep the whole grid), and a solve's fewest
 };
+
+// Grouped solves running on the device (those with a share).  A solve alone
+// has the device to itself, up to three blocks an SM, most of them waiting; where
+// handles are used by threads of their own, one solve's waiting blocks would
+// keep the others' off the SMs, so that the warps of blocks beyond an equal
+// share leave after one task, and the next kernel is not let in early.  (Handles
+// of idim 24..96, FP32, a thread each, ms until each has made an application: 24
+// of them 18.2 with whole grids, 6.7 so, 7.2 with level-by-level solves; 8 of them
+// 7.4, 4.0, 5.9; 2 of them 1.6, 1.3, 2.3.  With shares of 1, 1.5, 2.5, 3 blocks an
+// SM instead of 2, the 24 took 8.3, 6.8, 6.2, 13.6 and the 8 took 4.5, 4.2, 4.2,
+// 5.6.  Leaving before any task cost a solve alone 1 %: the count's round trip.)
+static __device__ int g_grp_running;
 
 __device__ __forceinline__ void grp_vals(const double *p, double *v) {
   const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
@@ -105,22 +121,36 @@ __device__ __forceinline__ void grp_gate(const T *p, int lane, int lim, int *err
 
 template <typename T, int KC>
 __global__ void __launch_bounds__(256) k_trsv_grp(GrpArgs<T> a) {
-  pdl_enter();
+  const int lane = threadIdx.x & 31;
+  if (a.share == 0)
+    pdl_enter();
+  else
+    pdl_wait();  // the solve before it on the same handle no longer counts
   constexpr int R = 32 / KC;
   typedef typename Bits<T>::U U;
   const U sent = (U)Sentinel<T>::bits;
-  const int lane = threadIdx.x & 31, c = lane % KC, rs = lane / KC;
+  const int c = lane % KC, rs = lane / KC;
   const int K = a.K, ncb = a.ncb, ntask = a.m.ntask * ncb;
   const int lim = spin_limit();
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.ctr_reset = 0;
-  int pend = 0;
-  if (lane == 0) pend = atomicAdd(a.ctr, 1);
+  int pend = 0, running = 0;
+  if (lane == 0) {
+    pend = atomicAdd(a.ctr, 1);
+    if (a.share && blockIdx.x == 0 && threadIdx.x == 0)
+      running = atomicAdd(&g_grp_running, 1) + 1;
+    else if (a.share)
+      running = (int)ld_relaxed_u32(&g_grp_running);
+  }
   int k = __shfl_sync(0xffffffffu, pend, 0);
-  if (lane == 0) pend = atomicAdd(a.ctr, 1);
+  running = __shfl_sync(0xffffffffu, running, 0);
+  // (block 0 never leaves: all tasks are claimed)
+  const bool leaves = running > 1 && (int)blockIdx.x >= max(a.least, a.share / running);
+  if (a.share && running <= 1) pdl_launch();
+  if (lane == 0) pend = leaves ? INT_MAX : atomicAdd(a.ctr, 1);
   int4 d = k < ntask ? __ldg(a.m.desc + k / ncb) : make_int4(0, 0, 0, 0);
   while (k < ntask) {
     const int kn = __shfl_sync(0xffffffffu, pend, 0);
-    if (lane == 0) pend = atomicAdd(a.ctr, 1);
+    if (lane == 0) pend = leaves ? INT_MAX : atomicAdd(a.ctr, 1);
     const int4 dn = kn < ntask ? __ldg(a.m.desc + kn / ncb) : make_int4(0, 0, 0, 0);
     const int col = (k % ncb) * KC + c;
     const int lt = d.w & 255, row = rs >> lt, nsw = d.y & 0xffff, nsv = d.y >> 16;
@@ -188,6 +218,7 @@ __global__ void __launch_bounds__(256) k_trsv_grp(GrpArgs<T> a) {
     k = kn;
     d = dn;
   }
+  if (a.share && blockIdx.x == 0 && threadIdx.x == 0) atomicSub(&g_grp_running, 1);
 }
 
 }  // namespace mldg

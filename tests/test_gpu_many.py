@@ -1,6 +1,8 @@
-"""GPU: many systems at once: a batch of more systems than the SMs have room
-for, each with a few blocks of its grouped solves, equals the systems one by
-one bit for bit."""
+"""GPU: many systems at once, in a batch of more systems than the SMs have room
+for, and on threads of their own: however many blocks a grouped solve is left
+with, the results equal those of the systems one by one bit for bit."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -35,3 +37,32 @@ def test_batch_of_many(mld, orc, precision):
         assert it == it1 and r == r1 and r <= 1e-10
         assert np.array_equal(x, x1)
         assert np.linalg.norm(b - orc.spmv(a, x)) <= 2e-10 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_handles_on_threads(mld, orc, precision):
+    """Applications, transposed ones and blocks, on ten handles at once."""
+    sy = _systems(mld, orc, [30, 8, 24, 12, 31, 17, 28, 9, 33, 21], precision)
+    X = [np.random.default_rng(k).uniform(-1, 1, (3, a.nrows)) for k, (a, _, _) in enumerate(sy)]
+
+    def calls(h, x):
+        return [h.apply(x[0]), h.apply(x[1], trans="T"), h.apply_block(x.copy()), h.krylov("FCG", x[2].copy(), eps=1e-8)[0]]
+
+    ref = [calls(h, x) for (_, h, _), x in zip(sy, X)]
+    bad = []
+
+    def work(h, x, r):
+        try:
+            for _ in range(15):
+                if not all(np.array_equal(y, z) for y, z in zip(calls(h, x), r)):
+                    bad.append("differs")
+        except Exception as e:  # noqa: BLE001 (a thread's failure is reported below)
+            bad.append(repr(e))
+
+    th = [threading.Thread(target=work, args=(h, x, r)) for (_, h, _), x, r in zip(sy, X, ref)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad
+    assert all(np.array_equal(y, z) for (_, h, _), x, r in zip(sy, X, ref) for y, z in zip(calls(h, x), r))
