@@ -34,7 +34,8 @@ struct TriGroups {
 // part by position, dep the positions of the dependencies.  A group grows by
 // whole levels while it holds at most `budget` entries of V and W together,
 // no row of either has more than `row`, and every row of W has an absolute sum
-// of at most `growth` (a bound on ||L_gg^{-1}||); a single level is always a
+// of at most `growth` (a bound on ||L_gg^{-1}||, by which the errors of the
+// explicit inverse can exceed those of a substitution); a single level is always a
 // group (W = I, V = L).  The rows of a level are shared by the OpenMP threads;
 // idim=45's factors (91,125 rows of 3 entries; 10,978 of 14), N and T, take 35
 // ms on 16 cores.

@@ -26,16 +26,18 @@ def _lower(n, per_row, size, near, seed):
     return T
 
 
-def _plan(mld, T, budget, row, growth, ncols=1):
+def _plan(mld, T, budget, row, growth, ncols=1, fp32=0, rhs=None):
     f = mld.lib().mldg_grp_plan_check
     f.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_longlong, C.c_int,
                   C.c_double, C.c_int, C.c_void_p]
     n = T.shape[0]
     c = mld.CSR(T.indptr, T.indices, T.data, ncols=n).c()
-    rhs = np.random.default_rng(1).uniform(-1, 1, n)
+    if rhs is None:
+        rhs = np.random.default_rng(1).uniform(-1, 1, n)
     t = np.zeros(n)
     st = np.zeros(4, np.int64)
-    assert f(C.byref(c), 0, None, rhs.ctypes.data, t.ctypes.data, ncols, budget, row, growth, 0, st.ctypes.data) == 0
+    assert f(C.byref(c), 0, None, rhs.ctypes.data, t.ctypes.data, ncols, budget, row, growth, fp32,
+             st.ctypes.data) == 0
     return t, st
 
 
@@ -112,3 +114,36 @@ def test_threads_do_not_change_the_plan():
                           env=dict(os.environ, OMP_NUM_THREADS=k), capture_output=True, text=True, check=True).stdout
            for k in ("1", "2", "7")]
     assert out[0].count("[0,") == 2 and out[0] == out[1] == out[2]
+
+
+@pytest.mark.parametrize("fp32", [0, 1])
+@pytest.mark.parametrize("a", [0.99, -0.99])
+def test_row_sums_near_the_bound(mld, a, fp32):
+    """A chain with ||L^{-1}|| = 100 and a smooth solution.  W's rows sum 1 + .99 +
+    .99^2 + ..., 63.8 after 101 terms, 64.1 after 102: 101 levels a
+    group.  A group's x_g = W b - V x errs by at most 105 u (|W||b| + |V||x|) (101
+    terms of W, one of V, their roundings and the storage of b and x), which later
+    groups pass on as G^{-1}, G = diag(W) L."""
+    n, k = 404, 101
+    L = np.eye(n) + np.diag(np.full(n - 1, a), -1)
+    D = np.zeros((n, n))
+    for g in range(0, n, k):
+        D[g:g + k, g:g + k] = L[g:g + k, g:g + k]
+    W = np.linalg.inv(D)
+    assert 63 < np.abs(W).sum(1).max() <= 64
+    V = W @ (L - D)
+    b = L @ (np.sin(np.arange(n) / 50.0) + 1.5)
+    x = np.zeros(n, np.longdouble)
+    for i in range(n):
+        x[i] = b[i] - (np.longdouble(a) * x[i - 1] if i else 0)
+    t, st = _plan(mld, sp.diags([np.full(n - 1, a)], [-1]).tocsr(), 0, 0, 0.0, fp32=fp32, rhs=b)
+    assert st[0] == 0 and st[2] == n // k
+    u = 2.0 ** (-24 if fp32 else -53)
+    local = 105 * u * (np.abs(W) @ np.abs(b) + np.abs(V) @ np.abs(x).astype(float))
+    assert np.all(np.abs(t - x) <= np.abs(np.linalg.inv(W @ L)) @ local)
+
+
+def test_growing_chain(mld):
+    """1 + 3 + 9 + 27 = 40 <= 64 < 121: four levels a group, exactly."""
+    _, st = _plan(mld, sp.diags([np.full(59, 3.0)], [-1]).tocsr(), 10 ** 9, 10 ** 6, 0.0)
+    assert st[0] == 0 and st[2] == 15
