@@ -43,8 +43,9 @@ int mldg_blk_plan_check(const mldg_csr *T, int upper, const double *scale, const
 
 /* Builds the grouped plan (k_trsv_grp) of the strictly triangular factor T
  * (0-based CSR, n x n; upper != 0: an upper factor) for ncols columns (a power
- * of two up to 32), exactly as mldg_finalize would, and replays its warp tasks
- * in ticket order on one right-hand side: every position written once, every
+ * of two up to 32), as mldg_finalize does for a right-hand side in original
+ * order (the second factor of a pair reads the first one's positions instead),
+ * and replays its warp tasks in ticket order on one right-hand side: every position written once, every
  * index in range, every dependency written by an earlier group.
  * t = (I + T)^{-1} (scale o rhs) (scale may be NULL).  budget, row, growth:
  * entries per group, entries per row and bound on a row of the inverted

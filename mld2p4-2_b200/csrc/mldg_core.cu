@@ -467,10 +467,9 @@ struct DBlk {
 };
 
 // Grouped solve: entries of V and W per group, entries of a row, the bound on a
-// row of W, and the widest block of columns
-// of a narrow level.  A group's entries should stream
-// in about the time of its hand-off, which takes longer the more warps take
-// part: n/5 entries between these limits (solve pair at idim=40, 64,000 rows:
+// row of W, and the widest block of columns of a narrow level.  A group's
+// entries should stream in about the time of its hand-off, which takes longer
+// the more warps take part: n/5 entries between these limits (solve pair at idim=40, 64,000 rows:
 // 86 us with 50,000 and 100,000, 98 us with 200,000; idim=101, 1,030,301 rows:
 // 333 us with 200,000, 408 us with 100,000).  Blocks above eight columns
 // move 16 or 32 values an entry, so a group holds fewer entries, and levels of
@@ -953,14 +952,6 @@ static void kdispatch(int K, F &&f) {
   }
 }
 // the ELL triangular solve also serves the single-vector V-cycle (K = 1)
-// the same with one column (K = 1) too
-template <typename F>
-static void kdispatch1(int K, F &&f) {
-  if (K == 1)
-    f(std::integral_constant<int, 1>());
-  else
-    kdispatch(K, f);
-}
 template <typename F>
 static void kdispatch_ell(int K, F &&f) {
   if (K == 1)
@@ -1698,7 +1689,7 @@ struct EngineT : Engine {
     a.share = grp_blocks > 0 ? 0 : kGrpShareBlocks * nsm;
     a.least = kGrpBatchLeast;
     begin(MLDG_KERNEL_TRSV);
-    grp_dispatch(Kw, [&](auto kc) { 
+    grp_dispatch(Kw, [&](auto kc) {
       kl(k_trsv_grp<T, decltype(kc)::value>, grp_blocks > 0 ? std::min(g.grid, grp_blocks) : g.grid, 256, a);
     });
     const int64_t vec = (int64_t)g.n * Kw * (int64_t)sizeof(T) * (3 + (out ? 1 + (beta != T(0)) : 0));
@@ -4580,7 +4571,7 @@ static Engine *make_engine(Handle *h) {
     // ILU(0) levels with wide rows (a coarse level's, above eight entries a
     // row), which the cluster solve runs faster: the fill of a wide row grows
     // with its square (idim=101 level 1, 129,684 rows of 14 entries: 256 us a
-    // cluster solve, 290 us a grouped one; level 0, 3 entries: 356 -> 167 us).
+    // cluster solve, 290 us a grouped one; level 0, 3 entries: 356 -> 155 us).
     L.grp = want_grp && L.n > 0 && !dense_coarse &&
             (H.kind == MLDG_SMOOTHER_FBGS ||
              (H.kind == MLDG_SMOOTHER_BJAC &&

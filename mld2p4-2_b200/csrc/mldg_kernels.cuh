@@ -83,10 +83,11 @@ template <> struct Bits<float> {
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // A small grid lets the next kernel in before it waits itself; a grid of more
-// than four blocks per SM (of 148) only after it, as its own later blocks need
-// the SMs (idim=160 level 0 in FP16 operators, repeated: the residual 45 us
-// this way, 53 the other).
-__device__ __forceinline__ bool pdl_early() { return gridDim.x <= 592; }
+// than four blocks per SM (of the B200's 148) only after it, as its own later
+// blocks need the SMs (idim=160 level 0 in FP16 operators, repeated: the
+// residual 45 us this way, 53 the other).
+constexpr unsigned kPdlEarlyBlocks = 4 * 148;
+__device__ __forceinline__ bool pdl_early() { return gridDim.x <= kPdlEarlyBlocks; }
 __device__ __forceinline__ void pdl_begin() {
   if (pdl_early()) pdl_launch();
 }
@@ -445,24 +446,24 @@ __global__ void __launch_bounds__(256) k_spmv_sell(int nr, const int *__restrict
         nr, soff, sj, sv, [&](int j) { return __ldg(v + j); },
         [&](int row) { return spmv_ops<T, V>(row, b, out, a2, rs); },
         [&](int row, T s, const SpmvOps<T> &p) { out[row] = spmv_value<T, V>(s, p, a1, b != nullptr, a0, a2); });
-    return;
-  }
-  pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int ns = (nr + 31) >> 5;
-  for (int sl0 = warp * S; sl0 < ns; sl0 += nwarps * S) {
-    T acc[S];
-    sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane, [&](int j) { return __ldg(v + j); }, acc);
+  } else {
+    pdl_enter();
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int ns = (nr + 31) >> 5;
+    for (int sl0 = warp * S; sl0 < ns; sl0 += nwarps * S) {
+      T acc[S];
+      sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane, [&](int j) { return __ldg(v + j); }, acc);
 #pragma unroll
-    for (int q = 0; q < S; ++q) {
-      const int row = ((sl0 + q) << 5) + lane;
-      if (row < nr) {
-        T r = a1 * row_scaled<T, V>(acc[q], rs, row);
-        if (b) r = fma(a0, b[row], r);
-        if (a2 != T(0)) r = fma(a2, out[row], r);
-        out[row] = r;
+      for (int q = 0; q < S; ++q) {
+        const int row = ((sl0 + q) << 5) + lane;
+        if (row < nr) {
+          T r = a1 * row_scaled<T, V>(acc[q], rs, row);
+          if (b) r = fma(a0, b[row], r);
+          if (a2 != T(0)) r = fma(a2, out[row], r);
+          out[row] = r;
+        }
       }
     }
   }
@@ -591,29 +592,29 @@ __global__ void __launch_bounds__(256) k_jacobi_sell(int nr, const int *__restri
       sell_loop<T>(nr, soff, sj, sv, [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, ep, done);
     else
       sell_loop<T>(nr, soff, sj, sv, [&](int j) { return __ldg(ty + j); }, ep, done);
-    return;
-  }
-  pdl_enter();
-  const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  const int ns = (nr + 31) >> 5;
-  for (int sl0 = warp * S; sl0 < ns; sl0 += nwarps * S) {
-    T acc[S];
-    if (first == 2)
-      sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane, [&](int j) { return omega * __ldg(x + j); }, acc);
-    else if (first)
-      sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane,
-                          [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, acc);
-    else
-      sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane, [&](int j) { return __ldg(ty + j); }, acc);
+  } else {
+    pdl_enter();
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int nwarps = (gridDim.x * blockDim.x) >> 5;
+    const int ns = (nr + 31) >> 5;
+    for (int sl0 = warp * S; sl0 < ns; sl0 += nwarps * S) {
+      T acc[S];
+      if (first == 2)
+        sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane, [&](int j) { return omega * __ldg(x + j); }, acc);
+      else if (first)
+        sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane,
+                            [&](int j) { return omega * (__ldg(d + j) * __ldg(x + j)); }, acc);
+      else
+        sell_rows<T, CI, S>(soff, sj, sv, sl0, ns, lane, [&](int j) { return __ldg(ty + j); }, acc);
 #pragma unroll
-    for (int q = 0; q < S; ++q) {
-      const int row = ((sl0 + q) << 5) + lane;
-      if (row < nr)
-        out[row] = jac_row(d[row], x[row], row_scaled<T, V>(acc[q], rs, row),
-                           (!first && omega != T(1)) ? ty[row] : T(0), first != 0, omega, alpha, beta,
-                           beta != T(0) ? out[row] : T(0));
+      for (int q = 0; q < S; ++q) {
+        const int row = ((sl0 + q) << 5) + lane;
+        if (row < nr)
+          out[row] = jac_row(d[row], x[row], row_scaled<T, V>(acc[q], rs, row),
+                             (!first && omega != T(1)) ? ty[row] : T(0), first != 0, omega, alpha, beta,
+                             beta != T(0) ? out[row] : T(0));
+      }
     }
   }
 }
