@@ -480,20 +480,24 @@ constexpr int64_t kGrpBudgetMin = 50000, kGrpBudgetMax = 200000;
 constexpr int kGrpRow = 512;
 constexpr double kGrpGrowth = 64.0;
 constexpr int kGrpCols = 8, kGrpWide = 8;
-// Blocks per SM that the grouped solves of a batch of systems share by their
-// rows, and the fewest of a system: a small one of many, left with two, was
-// slower than its level-by-level solve.  ms at 2.5, 3, 4, 5, 6 blocks per SM, at
-// least two: 64 systems of idim 24..96 201, 180, 174, 165, 154 (unbounded 620);
-// eight of them 55, 53, 52, 59, 68; 24 of them 95, 88, 81, 87, 92.  At four per SM
-// and at least 2, 4, 6, 8, 10: the 64 systems 174, 136, 139, 141, 143 (by level,
-// before the grouped solves, 149-156); 64 of idim 24..44 38.0, 35.4, 32.4, 32.3,
-// 33.2 (by level 31.7); 128 of them 69, 56, 55, 56, 56 (by level 48); 64 of idim
-// 40..72 96, 89, 83, 85, 87 (by level 88).
-constexpr double kGrpBatchBlocks = 4.0;
-constexpr int kGrpBatchLeast = 6;
-// blocks per SM that solves share which run at once without a batch, as the
-// kernel finds them (g_grp_running)
-constexpr int kGrpShareBlocks = 2;
+// The grouped solves of a batch share by their rows the blocks that the device
+// has room for, of kGrpBatchThreads threads (20 warps an SM in FP64, 28 in FP32;
+// 16 and 24 in blocks of 256): with fewer the SMs idle, with more some solves'
+// blocks keep out others that they do not wait for.  A system has at least
+// kGrpBatchLeast: a small one of many, left with two blocks of 256, was slower
+// than its level-by-level solve.  Measured in FP32, ms for 64, 48, 24 and 8 systems
+// of idim 24..96 and 64 of idim 24..44: 134, 109, 77, 51 and 29.4; with 6/7 of the
+// room 137, 107, 76, 51, 29.1, with 8/7 143, 112, 80, 55, 30.1; in blocks of 256
+// with 2/3 of their room 167, 129, 85, 55, 34.0, with all of it 141, 109, 77, 51,
+// 29.8, with twice it 159, 130, 98, 75, 35.4; by level 150, 131, 105, 91, 31.7;
+// with no bound 620 for the 64.  FP64: 176, 135, 85, 51 and 37.9; by level 157,
+// 137, -, 96 and 34.2: many systems of 64-bit values are the one case where the
+// entries that the groups add cost more than their hand-offs save.
+constexpr int kGrpBatchThreads = 128, kGrpBatchLeast = 12;
+// Solves that run at once without a batch divide half of the room equally
+// (g_grp_running), each with at least this many blocks.
+constexpr double kGrpShare = 0.5;
+constexpr int kGrpShareLeast = 6;
 static int64_t grp_budget(int n, int K) {
   return K > kGrpCols ? kGrpBudgetMin / 2 : K > 1 ? kGrpBudgetMin : std::max(kGrpBudgetMin, std::min<int64_t>(kGrpBudgetMax, n / 5));
 }
@@ -637,7 +641,7 @@ static int64_t grp_emulate(const TriGroups &g, const GrpTasks<T> &m, int KC, con
 // column width.
 template <typename T>
 struct DGrp {
-  int n = 0, grid = 0;
+  int n = 0, grid = 0, room = 0;  // blocks of a solve, and those that the device has room for
   GrpMat<T> m{};
   int64_t slots = 0;  // stored entries, padding included
   int *orig = nullptr;
@@ -1046,6 +1050,7 @@ struct Engine {
   // most blocks of a grouped solve, 0 for no bound: while a batch of systems is
   // captured, whose solves share the SMs
   int grp_blocks = 0;
+  int grp_room = 0;  // blocks of a batch's one-column grouped solve that the device has room for
   bool pdl_on() const { return pdl && probe_kind == 0 && !prof; }
   template <typename... KArgs, typename... Args>
   void kl(void (*kern)(KArgs...), int grid, int block, Args... args) {
@@ -1686,11 +1691,15 @@ struct EngineT : Engine {
     a.ctr = G.ctr + 32 * s;
     a.ctr_reset = G.ctr + 32 * r;
     a.err = err;
-    a.share = grp_blocks > 0 ? 0 : kGrpShareBlocks * nsm;
-    a.least = kGrpBatchLeast;
+    a.share = grp_blocks > 0 ? 0 : (int)(kGrpShare * g.room);
+    a.least = kGrpShareLeast;
     begin(MLDG_KERNEL_TRSV);
     grp_dispatch(Kw, [&](auto kc) {
-      kl(k_trsv_grp<T, decltype(kc)::value>, grp_blocks > 0 ? std::min(g.grid, grp_blocks) : g.grid, 256, a);
+      if (grp_blocks > 0)
+        kl(k_trsv_grp<T, decltype(kc)::value>, std::min(g.grid * (256 / kGrpBatchThreads), grp_blocks),
+           kGrpBatchThreads, a);
+      else
+        kl(k_trsv_grp<T, decltype(kc)::value>, g.grid, 256, a);
     });
     const int64_t vec = (int64_t)g.n * Kw * (int64_t)sizeof(T) * (3 + (out ? 1 + (beta != T(0)) : 0));
     end(g.slots * (int64_t)(sizeof(T) + 4) + 16 * (int64_t)g.m.ntask + vec,
@@ -2256,14 +2265,19 @@ struct EngineT : Engine {
     // warps in flight: eight groups' tasks, so that a group's tasks have their
     // entries and older values loaded when the group before it is finished
     // (idim=101 level 0: 822 us for four solves with four groups, 680 with eight)
-    int nb = 0;
+    int nb = 0, nbatch = 0;
     grp_dispatch(Kw, [&](auto kc) {
       MLDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trsv_grp<T, decltype(kc)::value>, 256, 0));
     });
     const int ng = (int)hp.pl.gptr.size() - 1;
     const int64_t ntask = (int64_t)g.m.ntask * (Kw / KC), per = (ntask + ng - 1) / ng;
     const int64_t warps = std::max<int64_t>(32, std::min<int64_t>((Kw > kGrpCols ? 4 : 8) * per, ntask));
-    g.grid = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, (int64_t)std::max(nb, 1) * nsm));
+    g.room = std::max(nb, 1) * nsm;
+    if (Kw == 1) {
+      MLDG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nbatch, k_trsv_grp<T, 1>, kGrpBatchThreads, 0));
+      grp_room = std::max(nbatch, 1) * nsm;
+    }
+    g.grid = (int)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, g.room));
     if (std::getenv("MLDG_VERBOSE"))
       std::fprintf(stderr, "mldg: grp K=%d n=%d levels=%d groups=%d entries %lld slots %lld tasks %d grid %d occ %d\n", Kw, n,
                    t.nlevels, ng, (long long)hp.pl.entries, (long long)g.slots, g.m.ntask, g.grid, nb);
@@ -5705,7 +5719,7 @@ static void end_capture_quietly(cudaStream_t st) {
 // that the concurrent branches of the other systems need (64 systems at idim
 // 24..96: 185 ms with it, against 155 ms without).
 // The systems' grouped solves share the SMs by their rows: a solve alone keeps
-// up to three blocks an SM waiting, which 64 systems have no room for.
+// two or three blocks an SM waiting, which 64 systems have no room for.
 struct NoPdlScope {
   std::vector<std::pair<Engine *, bool>> saved;
   NoPdlScope(int nsys, Handle **hs) {
@@ -5714,7 +5728,7 @@ struct NoPdlScope {
     for (int i = 0; i < nsys; ++i) {
       saved.emplace_back(hs[i]->eng.get(), hs[i]->eng->pdl);
       hs[i]->eng->pdl = false;
-      hs[i]->eng->grp_blocks = std::max(kGrpBatchLeast, (int)(kGrpBatchBlocks * hs[i]->nsm * hs[i]->n0 / std::max(rows, 1.0)));
+      hs[i]->eng->grp_blocks = std::max(kGrpBatchLeast, (int)(hs[i]->eng->grp_room * (hs[i]->n0 / std::max(rows, 1.0))));
     }
   }
   ~NoPdlScope() {

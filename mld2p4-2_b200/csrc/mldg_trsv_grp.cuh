@@ -62,15 +62,17 @@ struct GrpArgs {
 };
 
 // Grouped solves running on the device (those with a share).  A solve alone
-// has the device to itself, up to three blocks an SM, most of them waiting; where
-// handles are used by threads of their own, one solve's waiting blocks would
-// keep the others' off the SMs, so that the warps of blocks beyond an equal
-// share leave after one task, and the next kernel is not let in early.  (Handles
-// of idim 24..96, FP32, a thread each, ms until each has made an application: 24
-// of them 18.2 with whole grids, 6.7 so, 7.2 with level-by-level solves; 8 of them
-// 7.4, 4.0, 5.9; 2 of them 1.6, 1.3, 2.3.  With shares of 1, 1.5, 2.5, 3 blocks an
-// SM instead of 2, the 24 took 8.3, 6.8, 6.2, 13.6 and the 8 took 4.5, 4.2, 4.2,
-// 5.6.  Leaving before any task cost a solve alone 1 %: the count's round trip.)
+// has the device to itself, two (FP64) or three (FP32) blocks an SM, most of them
+// waiting; where handles are used by threads of their own, one solve's waiting
+// blocks would keep the others' off the SMs, so that the warps of blocks beyond
+// an equal share leave after one task, and the next kernel is not let in early.
+// (Handles of idim 24..96, a thread each, ms until each has made an application:
+// 24 of them in FP32 18.2 with whole grids; 6.8, 7.9, 9.9 with 1.5, 2, 2.25 blocks
+// an SM shared; 7.2 with level-by-level solves; 16 of them 11.7; 5.3, 5.9, 6.9;
+// 6.4; 8 of them 7.4; 4.1, 4.1, 4.4; 6.1; 2 of them 1.6, 1.4 with 2, 2.3.  FP64: 24
+// of them 24.8; 8.0, 9.1, 12.7 with 1, 1.33, 1.5 blocks; 7.8; 16 of them 15.8;
+// 5.9, 6.9, 9.2; 6.7; 8 of them 9.0; 4.5, 4.6, 5.3; 6.4.  Leaving before any task
+// cost a solve alone 1 %: the count's round trip.)
 static __device__ int g_grp_running;
 
 __device__ __forceinline__ void grp_vals(const double *p, double *v) {
