@@ -72,8 +72,12 @@ struct GrpArgs {
 // 6.4; 8 of them 7.4; 4.1, 4.1, 4.4; 6.1; 2 of them 1.6, 1.4 with 2, 2.3.  FP64: 24
 // of them 24.8; 8.0, 9.1, 12.7 with 1, 1.33, 1.5 blocks; 7.8; 16 of them 15.8;
 // 5.9, 6.9, 9.2; 6.7; 8 of them 9.0; 4.5, 4.6, 5.3; 6.4.  Leaving before any task
-// cost a solve alone 1 %: the count's round trip.)
+// cost a solve alone 1 %: the count's round trip.)  One column only: the wider
+// blocks' kernels with the same lines compiled slower (a solve of 32 right-hand
+// sides at idim=64 45.9 -> 48.0 ms), so that they keep their whole grids.
 static __device__ int g_grp_running;
+template <int KC>
+constexpr bool kGrpShares = KC == 1;
 
 __device__ __forceinline__ void grp_vals(const double *p, double *v) {
   const double2 a = __ldg(reinterpret_cast<const double2 *>(p)), b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
@@ -123,31 +127,32 @@ __device__ __forceinline__ void grp_gate(const T *p, int lane, int lim, int *err
 
 template <typename T, int KC>
 __global__ void __launch_bounds__(256) k_trsv_grp(GrpArgs<T> a) {
-  const int lane = threadIdx.x & 31;
-  if (a.share == 0)
-    pdl_enter();
-  else
+  if (kGrpShares<KC> && a.share)
     pdl_wait();  // the solve before it on the same handle no longer counts
+  else
+    pdl_enter();
   constexpr int R = 32 / KC;
   typedef typename Bits<T>::U U;
   const U sent = (U)Sentinel<T>::bits;
-  const int c = lane % KC, rs = lane / KC;
+  const int lane = threadIdx.x & 31, c = lane % KC, rs = lane / KC;
   const int K = a.K, ncb = a.ncb, ntask = a.m.ntask * ncb;
   const int lim = spin_limit();
   if (blockIdx.x == 0 && threadIdx.x == 0) *a.ctr_reset = 0;
-  int pend = 0, running = 0;
-  if (lane == 0) {
-    pend = atomicAdd(a.ctr, 1);
-    if (a.share && blockIdx.x == 0 && threadIdx.x == 0)
-      running = atomicAdd(&g_grp_running, 1) + 1;
-    else if (a.share)
-      running = (int)ld_relaxed_u32(&g_grp_running);
-  }
+  int pend = 0;
+  if (lane == 0) pend = atomicAdd(a.ctr, 1);
+  bool leaves = false;
+  int running = 0;
+  if (kGrpShares<KC> && a.share && lane == 0)
+    running = blockIdx.x == 0 && threadIdx.x == 0 ? atomicAdd(&g_grp_running, 1) + 1
+                                                  : (int)ld_relaxed_u32(&g_grp_running);
   int k = __shfl_sync(0xffffffffu, pend, 0);
-  running = __shfl_sync(0xffffffffu, running, 0);
-  // (block 0 never leaves: all tasks are claimed)
-  const bool leaves = running > 1 && (int)blockIdx.x >= max(a.least, a.share / running);
-  if (a.share && running <= 1) pdl_launch();
+  if (kGrpShares<KC> && a.share) {
+    running = __shfl_sync(0xffffffffu, running, 0);
+    if (running <= 1)
+      pdl_launch();
+    else  // (block 0 never leaves: all tasks are claimed)
+      leaves = (int)blockIdx.x >= max(a.least, a.share / running);
+  }
   if (lane == 0) pend = leaves ? INT_MAX : atomicAdd(a.ctr, 1);
   int4 d = k < ntask ? __ldg(a.m.desc + k / ncb) : make_int4(0, 0, 0, 0);
   while (k < ntask) {
@@ -220,7 +225,7 @@ __global__ void __launch_bounds__(256) k_trsv_grp(GrpArgs<T> a) {
     k = kn;
     d = dn;
   }
-  if (a.share && blockIdx.x == 0 && threadIdx.x == 0) atomicSub(&g_grp_running, 1);
+  if (kGrpShares<KC> && a.share && blockIdx.x == 0 && threadIdx.x == 0) atomicSub(&g_grp_running, 1);
 }
 
 }  // namespace mldg
