@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(256) k_trsv_grp(GrpArgs<T> a) {
     running = blockIdx.x == 0 && threadIdx.x == 0 ? atomicAdd(&g_grp_running, 1) + 1
                                                   : (int)ld_relaxed_u32(&g_grp_running);
   int k = __shfl_sync(0xffffffffu, pend, 0);
+  int4 d = k < ntask ? __ldg(a.m.desc + k / ncb) : make_int4(0, 0, 0, 0);
   if (kGrpShares<KC> && a.share) {
     running = __shfl_sync(0xffffffffu, running, 0);
     if (running <= 1)
@@ -154,7 +155,6 @@ __global__ void __launch_bounds__(256) k_trsv_grp(GrpArgs<T> a) {
       leaves = (int)blockIdx.x >= max(a.least, a.share / running);
   }
   if (lane == 0) pend = leaves ? INT_MAX : atomicAdd(a.ctr, 1);
-  int4 d = k < ntask ? __ldg(a.m.desc + k / ncb) : make_int4(0, 0, 0, 0);
   while (k < ntask) {
     const int kn = __shfl_sync(0xffffffffu, pend, 0);
     if (lane == 0) pend = leaves ? INT_MAX : atomicAdd(a.ctr, 1);
