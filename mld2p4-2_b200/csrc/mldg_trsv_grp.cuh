@@ -8,7 +8,7 @@
 // with one hand-off per group.  The price is fill: V and W hold more entries
 // than L, streamed once each.  Measured against the level-by-level solve it
 // replaced (us a solve, FP64): 4,096 rows, 46 levels in about 5 groups, 39 -> 18;
-// 1,030,301 rows, 301 levels in 88 groups (11 entries a row instead of 3),
+// 1,030,301 rows, 301 levels in 87 groups (11 entries a row instead of 3),
 // 356 -> 155; a Gauss-Seidel factor of 15,850 wide rows, 207 -> 100.  A group
 // costs 1.5-3 us, round trips of polls and gathers, where its bytes would
 // stream in under 0.5: a grid barrier a group instead (one cooperative kernel a
